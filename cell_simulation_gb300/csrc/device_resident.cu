@@ -10,13 +10,11 @@ namespace cellsim {
 namespace {
 
 constexpr int NT = RESIDENT_THREADS;
-constexpr int NSSA = RESIDENT_SSA_WARPS;
 
 // Byte offsets of a block's shared-memory areas, each 16-byte aligned.
 struct ResidentLayout {
     size_t cnt;    // [16] list lengths and counts, then PD_N diagnostic counters
     size_t thr;    // [thr_words] threshold table
-    size_t ws;     // [NSSA][SSA_WARP_SCRATCH] the SSA scratch of the warps that run the SSA
     size_t mark0, mark1;  // [vmax / 32] bitmaps: the voxel is on the current / the other work list
     size_t code;   // [vmax] region code (id + 1) of every voxel
     size_t dec;    // [vmax] move decisions of the current axis, valid for the voxels on the work
@@ -38,7 +36,6 @@ __host__ __device__ inline ResidentLayout resident_layout(int K, uint64_t vmax, 
     const size_t mark_words = (size_t)((vmax + 31) / 32);
     L.cnt = take(o, sizeof(uint32_t) * (16 + PD_N));
     L.thr = take(o, sizeof(uint32_t) * thr_words);
-    L.ws = take(o, sizeof(float) * (size_t)SSA_WARP_SCRATCH * NSSA);
     L.mark0 = take(o, sizeof(uint32_t) * mark_words);
     L.mark1 = take(o, sizeof(uint32_t) * mark_words);
     L.code = take(o, (size_t)vmax);
@@ -252,17 +249,14 @@ __global__ void __launch_bounds__(NT, 1) resident_frames_kernel(const __grid_con
         }
         __syncthreads();
         const uint32_t np = *n_pend;
-        if (warp < (uint32_t)NSSA) {
-            float* const ws = reinterpret_cast<float*>(sm + L.ws) + (size_t)warp * SSA_WARP_SCRATCH;
-            for (uint32_t q = warp; q < np; q += NSSA) {
-                const uint32_t v = dec[q];
-                Vox<K> r = cur[v];
-                const uint32_t rv = P.reservoir ? (uint32_t)P.reservoir[rd.base + v] : 0u;
-                const uint32_t w3 = d_philox(v, fr, 0u, 0u, k0, k1).w;
-                react_voxel_warp<K>(r, rv, v, fr, k0, k1, rd.rate_mult, ci, P.T, nullptr, counts, s_diag, w3, ws);
-                if (lane == 0u) cur[v] = r;
-                __syncwarp();
-            }
+        for (uint32_t q = warp; q < np; q += NT / 32) {
+            const uint32_t v = dec[q];
+            Vox<K> r = cur[v];
+            const uint32_t rv = P.reservoir ? (uint32_t)P.reservoir[rd.base + v] : 0u;
+            const uint32_t w3 = d_philox(v, fr, 0u, 0u, k0, k1).w;
+            react_voxel_warp<K>(r, rv, v, fr, k0, k1, rd.rate_mult, P.T, nullptr, counts, s_diag, w3);
+            if (lane == 0u) cur[v] = r;
+            __syncwarp();
         }
         if (all_react) {
             // reactions may fill empty voxels: the lists and marks start afresh from the lattice

@@ -508,8 +508,7 @@ __device__ __forceinline__ void stream_group(const StreamParams& SP, const WarpA
         }
         __syncwarp();
         if constexpr (PP == 3) {
-            // the SSA of the voxels this warp kept, by the whole warp (react_voxel_warp, its
-            // scratch in the list's storage), then what pass 3 does for a quiet voxel: the store,
+            // the SSA of the voxels this warp kept, by the whole warp (react_voxel_warp), then what pass 3 does for a quiet voxel: the store,
             // the occupancy bit and the next frame's x-decisions
             const uint32_t np = pend[0];
             if (np != 0u) {
@@ -533,9 +532,8 @@ __device__ __forceinline__ void stream_group(const StreamParams& SP, const WarpA
                     const uint2 f_yk = fpair(F_Y, (int)i), f_vc = fpair(F_VROW, (int)i);
                     const int yy = (int)f_yk.x, zz = 32 * (int)f_yk.y + (int)(pt.w & 31u);
                     const uint32_t v = f_vc.x + (uint32_t)zz;
-                    react_voxel_warp<K>(r, pt.y, v, frame, k0, k1, rd.rate_mult, rd.counts_index, P.T, nullptr,
-                                        P.counts + (size_t)rd.counts_index * S1, s_diag, pt.x,
-                                        reinterpret_cast<float*>(list));
+                    react_voxel_warp<K>(r, pt.y, v, frame, k0, k1, rd.rate_mult, P.T, nullptr,
+                                        P.counts + (size_t)rd.counts_index * S1, s_diag, pt.x);
                     if (lane == 0 && !vox_empty<K>(r)) {
                         st_vox_g<K>(dst + (rd.base + v) * K, r);
                         atomicOr(acc + i, bit);

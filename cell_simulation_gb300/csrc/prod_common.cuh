@@ -87,6 +87,7 @@ struct ProdTables {
     const uint32_t* quiet;            // [n_rep][S1][QS]: a voxel without reservoir holding one particle of
                                       // species p (q = 0), or one of p and one of q, has no reaction event
                                       // in the frame when (B(v,0)[3] >> 8) + 1 <= quiet[p][q]
+    const uint32_t* quiet_n;          // [n_rep][17]: quiet for any n particles (n <= 16)
     uint32_t QS;                      // S1 when two-particle entries are tabulated, else 1
     const float* g23;                 // [n_rep][2]: summed second- and third-order rates (times the
                                       // replicate's multiplier), for the propensity bound of fuller voxels
@@ -249,13 +250,17 @@ __device__ __forceinline__ Vox<K> combine(const Vox<K>& own, uint32_t down, cons
         uint32_t sl = (room_h + ((v_hi + frame + sweep) & 1u)) >> 1;
         out_p = lowest_bits(out_p, sl);
     }
-    uint32_t keep = ((1u << n_self) - 1u) & ~(out_m | out_p);
-    Vox<K> r = vox_zero<K>();
-    uint32_t j = 0;
-    while (keep) {
-        uint32_t s = __ffs(keep) - 1;
-        keep &= keep - 1;
-        vox_or<K>(r, j++, vox_get<K>(own, s));
+    Vox<K> r = own;
+    uint32_t j = n_self;
+    if (out_m | out_p) {
+        uint32_t keep = ((1u << n_self) - 1u) & ~(out_m | out_p);
+        r = vox_zero<K>();
+        j = 0;
+        while (keep) {
+            uint32_t s = __ffs(keep) - 1;
+            keep &= keep - 1;
+            vox_or<K>(r, j++, vox_get<K>(own, s));
+        }
     }
     while (acc_lo) {
         uint32_t s = __ffs(acc_lo) - 1;
@@ -481,159 +486,96 @@ __device__ __forceinline__ bool react_voxel_inline(Vox<K>& c, uint32_t resv, uin
     return fired;
 }
 
-// Index of set bit k (0-based) of the 128-bit mask (m0, m1); k < popcount.
-__device__ __forceinline__ int nth_bit(unsigned long long m0, unsigned long long m1, uint32_t k) {
-    uint32_t off = 0u;
-    uint32_t p0 = (uint32_t)__popcll(m0);
-    unsigned long long m = m0;
-    if (k >= p0) {
-        k -= p0;
-        m = m1;
-        off = 64u;
+// Removes one particle of species s (present) from a voxel of n: the last particle takes its slot.
+template <int K>
+__device__ __forceinline__ void vox_remove(Vox<K>& c, uint32_t s, uint32_t n) {
+    const uint64_t ones = 0x0101010101010101ull, rep = ones * s;
+    uint64_t x = c.w[0] ^ rep;
+    uint64_t z = (x - ones) & ~x & (ones << 7);  // the lowest set bit marks the first byte equal to s
+    uint32_t i = 0u;
+    if (K == 16 && z == 0ull) {
+        x = c.w[K / 8 - 1] ^ rep;
+        z = (x - ones) & ~x & (ones << 7);
+        i = 8u;
     }
-    uint32_t w = (uint32_t)m, pl = (uint32_t)__popc(w);
-    if (k >= pl) {
-        k -= pl;
-        w = (uint32_t)(m >> 32);
-        off += 32u;
-    }
-#pragma unroll
-    for (uint32_t sh = 16u; sh; sh >>= 1) {
-        const uint32_t c = (uint32_t)__popc(w & ((1u << sh) - 1u));
-        if (k >= c) {
-            k -= c;
-            w >>= sh;
-            off += sh;
-        }
-    }
-    return (int)off;
+    i += (uint32_t)(__ffsll((long long)z) - 1) >> 3;
+    const uint32_t last = vox_get<K>(c, n - 1u);
+    vox_set<K>(c, i, last);
+    vox_set<K>(c, n - 1u, 0u);
 }
-
-// Byte positions [a, b) of a 64-bit word (0 <= a, b <= 8) as a bit mask.
-__device__ __forceinline__ uint64_t byte_run_mask(int a, int b) {
-    a = min(max(a, 0), 8);
-    b = min(max(b, 0), 8);
-    if (b <= a) return 0ull;
-    const uint64_t hi = b == 8 ? ~0ull : (1ull << (8 * b)) - 1ull;
-    return hi & ~((1ull << (8 * a)) - 1ull);  // a < 8 here
-}
-
-// Words of the per-warp shared scratch react_voxel_warp uses (1408 bytes).
-constexpr int SSA_WARP_SCRATCH = 352;
 
 // The SSA of react_voxel_inline run by a whole warp: every lane calls it with
-// the same voxel and gets the same result.  The warp works on the voxel's
-// species histogram (in its shared scratch `ws`) instead of its slots: every
-// quantity of the SSA depends on the counts alone, and the content it returns
-// is rewritten species-major as react_voxel_inline's is.  Lane l owns
-// reactions l, l + 32, ...: the candidates' propensities go to their rank in
-// index order, lane 0 forms the running sums in that order (binary32 and, when
-// the selection needs it, binary64) exactly as react_voxel_inline does, and
-// the selected candidate is the first whose running sum exceeds the target (a
-// ballot over the stored binary32 sums; lane 0 scans the binary64 ones).  An
-// event's change list is applied one entry per lane, its species deltas added
-// to s_delta (shared) or, when that is null, to the global counts row
-// g_counts.  So every result, and so the lattice, equals react_voxel_inline's.
+// the same voxel and gets the same result.  It is a serial chain that other
+// work often waits for, so it is laid out for latency: the voxel's content
+// stays in every lane's registers (counts by byte compares, no histogram in
+// memory), lane l evaluates reactions l, l + 32, ..., and the running sums are
+// formed in index order by one shuffle and one add per candidate, each
+// candidate's lane keeping its own (binary32 and, when the selection needs it,
+// binary64) exactly as react_voxel_inline forms them.  The selected candidate
+// is the first whose running sum exceeds the target (a ballot).  An event's
+// change list is applied to the content, its species deltas added to s_delta
+// (shared) or, when that is null, to the global counts row g_counts.  The SSA of
+// one voxel with one event (GB300, the stiff 12-species network): 12.0k cycles
+// with the histogram and sums in shared memory, see react_voxel_warp's users.
 template <int K>
 __device__ __forceinline__ bool react_voxel_warp(Vox<K>& c, uint32_t resv, uint32_t v, uint32_t frame, uint32_t k0,
-                                                 uint32_t k1, float mult, uint32_t rep, const ProdTables& T,
-                                                 int32_t* s_delta, unsigned long long* g_counts, uint32_t* s_diag,
-                                                 uint32_t w3, float* ws) {
+                                                 uint32_t k1, float mult, const ProdTables& T, int32_t* s_delta,
+                                                 unsigned long long* g_counts, uint32_t* s_diag, uint32_t w3) {
+    constexpr int CH = 4;  // chunks of 32 reactions (R <= 128)
     const uint32_t lane = threadIdx.x & 31u;
-    if (T.R == 0) return false;
+    const uint32_t R = T.R;
+    if (R == 0) return false;
     if (lane == 0u) atomicAdd(s_diag + PD_SSA_VOXELS, 1u);
-    float* const a_s = ws;                                      // [128] propensities by candidate rank
-    float* const p_s = ws + 128;                                // [128] their binary32 running sums
-    uint8_t* const hist = reinterpret_cast<uint8_t*>(ws + 256);  // [256] particles per species
-    uint8_t* const r_s = reinterpret_cast<uint8_t*>(ws + 320);   // [128] reaction of each rank
-    const uint32_t S1 = T.S1, R = T.R;
+    const uint32_t* const rmask = reinterpret_cast<const uint32_t*>(T.rmask);  // 4 words per species
+    const uint32_t zm[CH] = {(uint32_t)T.zmask[0], (uint32_t)(T.zmask[0] >> 32), (uint32_t)T.zmask[1],
+                             (uint32_t)(T.zmask[1] >> 32)};
     uint32_t n = vox_n<K>(c);
-    for (uint32_t s = lane; s < S1; s += 32u) hist[s] = s ? (uint8_t)vox_count<K>(c, s) : (uint8_t)0;
-    __syncwarp();
     double td = 0.0;
     float tf = 0.0f;
     bool fired = false;
     uint32_t ev = 0;
     for (; ev < T.max_events; ev++) {
-        // candidates: reactions with a reactant present (or none at all)
-        unsigned long long c0 = 0ull, c1 = 0ull;
-        for (uint32_t s = 1u + lane; s < S1; s += 32u)
-            if (hist[s] > 0) {
-                c0 |= tab_ld(T.rmask + 2 * s);
-                c1 |= tab_ld(T.rmask + 2 * s + 1);
-            }
-        c0 = ((unsigned long long)__reduce_or_sync(0xffffffffu, (uint32_t)(c0 >> 32)) << 32) |
-             __reduce_or_sync(0xffffffffu, (uint32_t)c0);
-        c1 = ((unsigned long long)__reduce_or_sync(0xffffffffu, (uint32_t)(c1 >> 32)) << 32) |
-             __reduce_or_sync(0xffffffffu, (uint32_t)c1);
-        c0 |= T.zmask[0];
-        c1 |= T.zmask[1];
-        if (resv) {
-            c0 |= tab_ld(T.rmask + 2 * resv);
-            c1 |= tab_ld(T.rmask + 2 * resv + 1);
-        }
-        const uint32_t p0 = (uint32_t)__popcll(c0);
-        const uint32_t nc = p0 + (uint32_t)__popcll(c1);
-        uint32_t bmax = 0u, bmin = 0x7f800000u;  // bit patterns of positive binary32 order like the values
-        for (uint32_t r = lane; r < R; r += 32u) {
-            const bool cand = r < 64u ? ((c0 >> r) & 1ull) != 0ull : ((c1 >> (r - 64u)) & 1ull) != 0ull;
-            if (!cand) continue;
-            const uint32_t rank = r < 64u ? (uint32_t)__popcll(c0 & ((1ull << r) - 1ull))
-                                          : p0 + (uint32_t)__popcll(c1 & ((1ull << (r - 64u)) - 1ull));
-            // the propensity of react_voxel_inline, from the histogram
-            const uint8_t* re = T.rx_reactants + 3 * r;
-            const uint32_t sp[3] = {tab_ld(re), tab_ld(re + 1), tab_ld(re + 2)};
-            uint32_t ff = 1u;
-            bool zero = false;
+        const uint32_t q_l = lane < n ? vox_get<K>(c, lane) : 0u;
+        uint32_t cm[CH];  // candidates: reactions with a reactant present (or none at all)
+        float a[CH], p[CH];
+        float run = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 3; j++) {
-                const uint32_t q = sp[j];
-                if (q == 0u) continue;
-                uint32_t m = 0u;
+        for (int h = 0; h < CH; h++) {
+            cm[h] = 0u;
+            a[h] = p[h] = 0.0f;
+            if (32u * h < R) {
+                uint32_t m = lane < n ? tab_ld(rmask + 4 * q_l + h) : 0u;
+                m = __reduce_or_sync(0xffffffffu, m) | zm[h];
+                if (resv) m |= tab_ld(rmask + 4 * resv + h);
+                cm[h] = m;
+                if ((m >> lane) & 1u) {
+                    const uint32_t r = 32u * h + lane;
+                    const uint8_t* re = T.rx_reactants + 3 * r;
+                    const uint32_t sp[3] = {tab_ld(re), tab_ld(re + 1), tab_ld(re + 2)};
+                    const float rate = tab_ld(T.rx_rate + r);
+                    uint32_t ff = 1u;
+                    bool zero = false;
 #pragma unroll
-                for (int i = 0; i < j; i++) m += sp[i] == q;
-                const uint32_t cnt = q == resv ? 1u : (uint32_t)hist[q];
-                if (cnt <= m) zero = true;
-                else ff *= cnt - m;
-            }
-            const float a = zero ? 0.0f : __fmul_rn(__fmul_rn(tab_ld(T.rx_rate + r), mult), (float)ff);
-            a_s[rank] = a;
-            r_s[rank] = (uint8_t)r;
-            if (a > 0.0f) {
-                bmax = max(bmax, __float_as_uint(a));
-                bmin = min(bmin, __float_as_uint(a));
-            }
-        }
-        __syncwarp();
-        if (lane == 0u) {
-            float run = 0.0f;
-            for (uint32_t k = 0; k < nc; k++) {
-                run = __fadd_rn(run, a_s[k]);
-                p_s[k] = run;
-            }
-        }
-        __syncwarp();
-        const uint32_t rounds = (nc + 31u) >> 5;
-        float a0, amax, amin;
-        if (resv == 0u && n <= 1u) {
-            uint32_t sole = 0u;  // the species of the voxel's one particle
-            if (n == 1u)
-                for (uint32_t base = 0; base < S1; base += 32u) {
-                    const uint32_t b = __ballot_sync(0xffffffffu, base + lane < S1 && hist[base + lane] > 0);
-                    if (b) {
-                        sole = base + (uint32_t)__ffs((int)b) - 1u;
-                        break;
+                    for (int j = 0; j < 3; j++) {
+                        const uint32_t q = sp[j];
+                        if (q == 0u) continue;
+                        uint32_t dup = 0u;
+#pragma unroll
+                        for (int i = 0; i < j; i++) dup += sp[i] == q;
+                        const uint32_t cnt = q == resv ? 1u : vox_count<K>(c, q);
+                        if (cnt <= dup) zero = true;
+                        else ff *= cnt - dup;
                     }
+                    a[h] = zero ? 0.0f : __fmul_rn(__fmul_rn(rate, mult), (float)ff);
                 }
-            const float* o = T.one + ((size_t)rep * S1 + sole) * 3;
-            a0 = tab_ld(o);
-            amax = tab_ld(o + 1);
-            amin = tab_ld(o + 2);
-        } else {
-            a0 = nc ? p_s[nc - 1u] : 0.0f;
-            amax = __uint_as_float(__reduce_max_sync(0xffffffffu, bmax));
-            amin = __uint_as_float(__reduce_min_sync(0xffffffffu, bmin));
+                for (uint32_t b = m; b; b &= b - 1u) {
+                    const int k = __ffs((int)b) - 1;
+                    run = __fadd_rn(run, __shfl_sync(0xffffffffu, a[h], k));
+                    if ((int)lane == k) p[h] = run;
+                }
+            }
         }
+        const float a0 = run;
         if (!(a0 > 0.0f)) break;
         U4 ph{0u, 0u, 0u, 0u};
         uint32_t w1 = w3;
@@ -653,44 +595,59 @@ __device__ __forceinline__ bool react_voxel_warp(Vox<K>& c, uint32_t resv, uint3
         if (ev == 0u) ph = d_philox(v, frame, 0x80000000u, 0u, k0, k1);
         const uint32_t w2 = ph.y;
         float u2 = __fmul_rn((float)(w2 >> 8), 0x1p-24f);
-        bool use64 = (T.precision == 2) || (T.precision == 0 && amax > __fmul_rn(1e6f, amin));
+        bool use64 = T.precision == 2;
+        if (T.precision == 0) {
+            uint32_t bmax = 0u, bmin = 0x7f800000u;  // bit patterns of positive binary32 order like the values
+#pragma unroll
+            for (int h = 0; h < CH; h++)
+                if (a[h] > 0.0f) {
+                    bmax = max(bmax, __float_as_uint(a[h]));
+                    bmin = min(bmin, __float_as_uint(a[h]));
+                }
+            bmax = __reduce_max_sync(0xffffffffu, bmax);
+            bmin = __reduce_min_sync(0xffffffffu, bmin);
+            use64 = __uint_as_float(bmax) > __fmul_rn(1e6f, __uint_as_float(bmin));
+        }
         // first candidate whose running sum exceeds the target; else the last one with a positive
         // propensity (the sequential scan's last_pos)
-        int idx = -1;
+        int sel = -1;
         if (!use64) {
             const float target = __fmul_rn(u2, a0);
-            for (uint32_t q = 0; q < rounds && idx < 0; q++) {
-                const uint32_t k = q * 32u + lane;
-                const uint32_t b = __ballot_sync(0xffffffffu, k < nc && target < p_s[k]);
-                if (b) idx = (int)(q * 32u) + __ffs((int)b) - 1;
-            }
+#pragma unroll
+            for (int h = 0; h < CH; h++)
+                if (32u * h < R && sel < 0) {
+                    const uint32_t b = __ballot_sync(0xffffffffu, ((cm[h] >> lane) & 1u) && target < p[h]);
+                    if (b) sel = 32 * h + __ffs((int)b) - 1;
+                }
         } else {
-            if (lane == 0u) {
-                atomicAdd(s_diag + PD_FP64_SEL, 1u);
-                double a0d = 0.0;
-                for (uint32_t k = 0; k < nc; k++) a0d = __dadd_rn(a0d, (double)a_s[k]);
-                const double target = __dmul_rn((double)u2, a0d);
-                double run = 0.0;
-                for (uint32_t k = 0; k < nc; k++) {
-                    run = __dadd_rn(run, (double)a_s[k]);
-                    if (target < run) {
-                        idx = (int)k;
-                        break;
-                    }
+            if (lane == 0u) atomicAdd(s_diag + PD_FP64_SEL, 1u);
+            double a0d = 0.0, pd[CH];
+#pragma unroll
+            for (int h = 0; h < CH; h++) {
+                pd[h] = 0.0;
+                for (uint32_t b = cm[h]; b; b &= b - 1u) {
+                    const int k = __ffs((int)b) - 1;
+                    a0d = __dadd_rn(a0d, (double)__shfl_sync(0xffffffffu, a[h], k));
+                    if ((int)lane == k) pd[h] = a0d;
                 }
             }
-            idx = __shfl_sync(0xffffffffu, idx, 0);
+            const double target = __dmul_rn((double)u2, a0d);
+#pragma unroll
+            for (int h = 0; h < CH; h++)
+                if (32u * h < R && sel < 0) {
+                    const uint32_t b = __ballot_sync(0xffffffffu, ((cm[h] >> lane) & 1u) && target < pd[h]);
+                    if (b) sel = 32 * h + __ffs((int)b) - 1;
+                }
         }
-        if (idx < 0) {
-            for (int q = (int)rounds - 1; q >= 0 && idx < 0; q--) {
-                const uint32_t k = (uint32_t)q * 32u + lane;
-                const uint32_t b = __ballot_sync(0xffffffffu, k < nc && a_s[k] > 0.0f);
-                if (b) idx = q * 32 + 31 - __clz((int)b);
-            }
+        if (sel < 0) {
+#pragma unroll
+            for (int h = CH - 1; h >= 0; h--)
+                if (32u * h < R && sel < 0) {
+                    const uint32_t b = __ballot_sync(0xffffffffu, a[h] > 0.0f);
+                    if (b) sel = 32 * h + 31 - __clz((int)b);
+                }
         }
-        const uint32_t sel = idx >= 0 ? (uint32_t)r_s[idx] : 0u;
-        __syncwarp();  // the scratch is rewritten by the next event
-        if (idx < 0) break;
+        if (sel < 0) break;
         // the change list (distinct species, ending at the first zero), one entry per lane; the
         // voxel's reservoir species is skipped
         const uint32_t es = lane < 8u ? (uint32_t)tab_ld(T.rx_ch_sp + 8 * sel + lane) : 0u;
@@ -698,52 +655,47 @@ __device__ __forceinline__ bool react_voxel_warp(Vox<K>& c, uint32_t resv, uint3
         const uint32_t zb = __ballot_sync(0xffffffffu, lane < 8u && es == 0u);
         const uint32_t n_ent = zb ? (uint32_t)__ffs((int)zb) - 1u : 8u;
         const bool act = lane < n_ent && es != resv;
-        const int have = act ? hist[es] : 0;
-        const int total = (int)n + __reduce_add_sync(0xffffffffu, (uint32_t)(act ? ed : 0));
+        const int have = act ? (int)vox_count<K>(c, es) : 0;
+        const int total = (int)n + (int)__reduce_add_sync(0xffffffffu, (uint32_t)(act ? ed : 0));
         if (__any_sync(0xffffffffu, act && have + ed < 0) || total > (int)K) {
             if (lane == 0u) atomicAdd(s_diag + PD_REJECT_CAP, 1u);
             continue;
         }
         if (act) {
-            hist[es] = (uint8_t)(have + ed);
             if (s_delta) atomicAdd(s_delta + es, ed);
             else atomicAdd(g_counts + es, (unsigned long long)(long long)ed);
         }
-        __syncwarp();
-        n = (uint32_t)total;
+        // removals first, so that the content never exceeds K slots in between
+        const uint32_t acts = __ballot_sync(0xffffffffu, act);
+        for (uint32_t b = acts; b; b &= b - 1u) {
+            const int k = __ffs((int)b) - 1;
+            const uint32_t s = __shfl_sync(0xffffffffu, es, k);
+            for (int d = __shfl_sync(0xffffffffu, ed, k); d < 0; d++) vox_remove<K>(c, s, n--);
+        }
+        for (uint32_t b = acts; b; b &= b - 1u) {
+            const int k = __ffs((int)b) - 1;
+            const uint32_t s = __shfl_sync(0xffffffffu, es, k);
+            for (int d = __shfl_sync(0xffffffffu, ed, k); d > 0; d--) vox_or<K>(c, n++, s);
+        }
         if (lane == 0u) atomicAdd(s_diag + PD_EVENTS, 1u);
         fired = true;
     }
     if (ev == T.max_events && lane == 0u) atomicAdd(s_diag + PD_EVENT_CAP, 1u);
     if (fired) {
-        // species-major rewrite, ascending species id: lane l writes the run of species
-        // base + l at its exclusive prefix of the counts
-        uint64_t w[K / 8];
-#pragma unroll
-        for (int i = 0; i < K / 8; i++) w[i] = 0ull;
-        int off = 0;
-        for (uint32_t base = 0; base < S1; base += 32u) {
-            const uint32_t s = base + lane;
-            const int cnt = (s > 0u && s < S1) ? hist[s] : 0;
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)lane >= o) incl += u;
-            }
-            const int a = off + incl - cnt;
-            if (cnt > 0) {
-                const uint64_t rep8 = (uint64_t)s * 0x0101010101010101ull;
-#pragma unroll
-                for (int i = 0; i < K / 8; i++) w[i] |= rep8 & byte_run_mask(a - 8 * i, a + cnt - 8 * i);
-            }
-            off += __shfl_sync(0xffffffffu, incl, 31);
+        // species-major rewrite, ascending species id: lane l's particle at its rank
+        const uint32_t q = lane < n ? vox_get<K>(c, lane) : 0u;
+        uint32_t rank = 0u;
+        for (uint32_t j = 0; j < n; j++) {
+            const uint32_t o = vox_get<K>(c, j);
+            rank += o < q || (o == q && j < lane);
         }
         Vox<K> out;
 #pragma unroll
-        for (int i = 0; i < K / 8; i++)
-            out.w[i] = ((uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(w[i] >> 32)) << 32) |
-                       __reduce_or_sync(0xffffffffu, (uint32_t)w[i]);
+        for (int i = 0; i < K / 8; i++) {
+            const uint64_t w = lane < n && (int)(rank >> 3) == i ? (uint64_t)q << (8 * (rank & 7u)) : 0ull;
+            out.w[i] = ((uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(w >> 32)) << 32) |
+                       __reduce_or_sync(0xffffffffu, (uint32_t)w);
+        }
         c = out;
     }
     return fired;

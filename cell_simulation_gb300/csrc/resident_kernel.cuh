@@ -29,7 +29,6 @@
 namespace cellsim {
 
 constexpr int RESIDENT_THREADS = 512;
-constexpr int RESIDENT_SSA_WARPS = 8;  // the warps that run the SSA (1408 bytes of scratch each)
 
 struct ResidentParams {
     ProdParams P;          // tables, replicates, counts, diagnostics; P.src holds the call's first
