@@ -1149,7 +1149,8 @@ void ref_render_view(DeviceRef* d, int32_t view, int32_t slice_axis, uint32_t sl
     v.slice_axis = slice_axis;
     v.slice = slice;
     v.out = out_dev;
-    render_view_kernel<<<1024, 256, 0, d->stream>>>(v);
+    if (view == 0 && slice == 0u && (v.K == 8u || v.K == 16u)) launch_majority_view(v.K, v.slots, d->p.V, out_dev, d->stream);
+    else render_view_kernel<<<1024, 256, 0, d->stream>>>(v);
     CS_LAUNCH_CHECK();
     if (!out_device) CS_CUDA(cudaMemcpyAsync(out_host, out_dev, d->p.V * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
     CS_CUDA(cudaStreamSynchronize(d->stream));
