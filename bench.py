@@ -258,7 +258,13 @@ def describe_variant(i):
     if kind == 3:  # one block per replicate, every frame of a step call in one launch
         return {"index": i, "kind": "resident", "slots": k, "threads": nt, "multi_frame": True,
                 "launches_per_call": 1}
+    if kind == 4:  # one block per replicate keeps the list of its occupied voxels for a whole step call
+        return {"index": i, "kind": "resident", "lists": True, "slots": k, "threads": nt, "multi_frame": True,
+                "launches_per_call": 1}
     if kind == 2:
+        if ty == 2:  # sweeps in place over the voxels that change, decisions of all axes in one pass
+            return {"index": i, "kind": "stream", "in_place": True, "slots": k, "threads": nt,
+                    "passes_per_frame": tiling_launches()[i]}
         if ty == 1:  # the persistent form: every frame of a step call in one launch
             return {"index": i, "kind": "stream", "slots": k, "words_per_group": 32, "threads": nt,
                     "passes_per_frame": 2, "multi_frame": True, "launches_per_call": 1}
@@ -287,13 +293,15 @@ def launches_in_call(i, frames):
 def frame_kernels(desc):
     """The kernels of one frame of a variant, as named in the committed ncu summaries."""
     if desc["kind"] == "stream":
+        if desc.get("in_place"):
+            return ["inplace_line_kernel<0>", "inplace_line_kernel<1>", "inplace_row_kernel"]
         if desc.get("multi_frame"):
             return ["sweep_frames_kernel"]
         if desc["passes_per_frame"] == 2:
             return ["sweep_pass_kernel<1>", "sweep_pass_kernel<5>"]
         return ["sweep_pass_kernel<1>", "sweep_pass_kernel<2>", "sweep_pass_kernel<3>"]
     if desc["kind"] == "resident":
-        return ["resident_frames_kernel"]
+        return ["list_frames_kernel" if desc.get("lists") else "resident_frames_kernel"]
     return ["brick_step_kernel"] if desc["kind"] == "brick" else ["prod_step_kernel"]
 
 

@@ -34,6 +34,8 @@
 #include "cuda_check.h"
 #include "internal.h"
 #include "brick_kernel.cuh"
+#include "inplace_kernel.cuh"
+#include "lists_kernel.cuh"
 #include "prod_common.cuh"
 #include "prod_kernel.cuh"
 #include "resident_kernel.cuh"
@@ -52,8 +54,9 @@ typedef void (*ProdKernelFn)(ProdParams);
 // pools as large as its box finishes the spilled bricks in `sub` groups of
 // its own BX planes.  kind 2: the sweep stream, four barrier-free passes over
 // bitmap word groups (stream_kernel.cuh); `variant` indexes its compiled
-// launch shapes.
-enum { KIND_TILE = 0, KIND_BRICK = 1, KIND_STREAM = 2, KIND_RESIDENT = 3 };
+// launch shapes.  KIND_INPLACE: the in-place form of the sweep stream (inplace_kernel.cuh),
+// reported as kind 2 with TY = 2.  KIND_LISTS: the list form (lists_kernel.cuh).
+enum { KIND_TILE = 0, KIND_BRICK = 1, KIND_STREAM = 2, KIND_RESIDENT = 3, KIND_LISTS = 4, KIND_INPLACE = 5 };
 
 struct KernelCfg {
     int kind, K, TY, TZ, NT, BX;
@@ -73,6 +76,16 @@ static KernelCfg stream_cfg(int K, int variant) {
 // the resident form: one block per replicate, every frame of a step call in one launch
 static KernelCfg resident_cfg(int K) {
     return KernelCfg{KIND_RESIDENT, K, 0, 0, RESIDENT_THREADS, 0, nullptr, nullptr, -1, 0, 0};
+}
+
+// the in-place sweep stream, marked by TY = 2 (cs_tiling_describe)
+static KernelCfg inplace_cfg(int K) {
+    return KernelCfg{KIND_INPLACE, K, 2, 32, INPLACE_THREADS, 0, nullptr, nullptr, -1, 0, 0};
+}
+
+// the list form: one block per replicate, every frame of a step call in one launch
+static KernelCfg lists_cfg(int K) {
+    return KernelCfg{KIND_LISTS, K, 0, 0, 256, 0, nullptr, nullptr, -1, 0, 0};
 }
 
 template <int K, int TY, int TZ>
@@ -122,7 +135,7 @@ static const std::vector<KernelCfg>& all_cfgs() {
         // sweep stream: 256 threads, at least two / four blocks per SM (pass 3 of variants 2, 3: three, two)
         stream_cfg(16, 0), stream_cfg(16, 1), stream_cfg(8, 0), stream_cfg(8, 1), stream_cfg(16, 2), stream_cfg(8, 2),
         stream_cfg(16, 3), stream_cfg(8, 3),
-        // sweep stream with the Y and Z sweeps fused into one launch (rows of at most 32 words), at
+        // sweep stream with the Y and Z sweeps fused into one launch (edges of at most 1024 voxels), at
         // three / four blocks per SM
         stream_cfg(16, 4), stream_cfg(8, 4), stream_cfg(16, 5), stream_cfg(8, 5),
         // the fused stream as one persistent launch per step call (pass 1 and the fused pass of
@@ -131,6 +144,10 @@ static const std::vector<KernelCfg>& all_cfgs() {
         stream_cfg(16, 6), stream_cfg(8, 6), stream_cfg(16, 7), stream_cfg(8, 7),
         // lattices that fit in one block's shared memory: the resident form
         resident_cfg(16), resident_cfg(8),
+        // the in-place sweep stream (rows of at most 32 words)
+        inplace_cfg(16), inplace_cfg(8),
+        // lists of occupied voxels (replicates of a few hundred particles)
+        lists_cfg(16), lists_cfg(8),
     };
     return v;
 }
@@ -160,7 +177,7 @@ struct DeviceProd {
     DevBuf<float> rx_rate;
     DevBuf<unsigned long long> rmask;
     DevBuf<float> one;
-    DevBuf<uint32_t> quiet;
+    DevBuf<uint32_t> quiet, quiet_n;
     DevBuf<float> g23;
     DevBuf<float> a2;  // pair propensities (ProdTables::a2)
     DevBuf<WorkItem> spill;  // bricks handed from the brick pass to the second pass
@@ -181,6 +198,7 @@ struct DeviceProd {
     uint32_t n_groups = 0;
     DevBuf<uint4> rec[3];  // two parities; fused variants: x-, y- and z-decision records in 0, 1, 2
     DevBuf<uint32_t> sw[14];
+    DevBuf<uint32_t> uni;   // per bitmap word: voxels whose neighbours lie inside and share their code
     DevBuf<uint8_t> wcode;  // per bitmap word: uniform region code of its window, or 0 (single lattices)
     DevBuf<uint2> ssa_over;  // pass 3: per-warp lists of the voxels set aside for the warp's SSA
     // the multi-frame form: per group its four neighbours and the completion values of its last
@@ -201,6 +219,33 @@ struct DeviceProd {
     bool xdec_valid = false;
     uint64_t xdec_frame = 0, xdec_epoch = 0;
     int xdec_cur = 0, xdec_cfg = -1;
+    // the in-place form: units of its three launches (rep-major, offsets per replicate, most words of
+    // a unit), move decisions per axis, reacting voxels, voxels with a reservoir
+    DevBuf<LineUnit> units[3];
+    std::vector<uint32_t> unit_off[3];
+    uint32_t unit_words[3] = {0, 0, 0};
+    DevBuf<uint2> mv[3];
+    DevBuf<uint32_t> dec[3];
+    DevBuf<uint32_t> mul, react, resv_bits;
+    cudaGraphExec_t ip_graph[8] = {};  // of 1 .. kInplaceGraphFrames frames
+    int ip_graph_cur[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
+    // the list form: voxels, contents and lengths of every replicate's list (l_cap entries each), a
+    // host-visible word that it sets when a replicate outgrew its list; ls_state: the lattice is in the
+    // lists.  p_max: the most particles of a replicate, as last seen by the host.
+    DevBuf<uint32_t> l_xyz, l_n;
+    DevBuf<uint8_t> l_cont;
+    uint32_t l_cap = 0;
+    uint32_t* h_flag = nullptr;
+    bool ls_state = false;
+    uint64_t p_max = 0;
+    uint32_t one_code = 0;  // the region code of every voxel of a single lattice when they share one, else 0
+    DevBuf<uint8_t> spec;  // species of the voxels of one particle, 32 bytes per bitmap word
+    // ip_state: the lattice is in the form's own layout (occ[cur], mul, spec and, for voxels of two or
+    // more particles, slots[cur]); ip_valid: the decisions of its frame ip_frame (seed epoch ip_epoch)
+    // are in mv, dec and react.  Cleared by every other change of the lattice.  slots_stale: the other
+    // voxels of slots[cur] have not been written since (ensure_slots writes them).
+    bool ip_state = false, ip_valid = false, slots_stale = false;
+    uint64_t ip_frame = 0, ip_epoch = 0;
     uint64_t seed_epoch = 0;  // advanced whenever the Philox keys change
     uint64_t next_frame = 0;  // host copy of the frame number in stepbuf[cur]
     // stepbuf[cur] holds next_frame in stream order: it was uploaded, and every frame since wrote
@@ -227,7 +272,10 @@ struct DeviceProd {
         if (graph) cudaGraphExecDestroy(graph);
         for (cudaGraphExec_t g1 : graph1)
             if (g1) cudaGraphExecDestroy(g1);
+        for (cudaGraphExec_t g1 : ip_graph)
+            if (g1) cudaGraphExecDestroy(g1);
         if (h_counts) cudaFreeHost(h_counts);
+        if (h_flag) cudaFreeHost(h_flag);
         if (h_frames) cudaFreeHost(h_frames);
         for (cudaEvent_t e : frame_ev)
             if (e) cudaEventDestroy(e);
@@ -429,8 +477,10 @@ static void build_one_table(DeviceProd* d) {
     // reactions whose reactants are exactly p and q, twice for p == q (n(n-1) counts each
     // unordered pair of p twice), rounded up; tabulated beside the two-particle thresholds
     d->T.a2 = nullptr;
+    std::vector<float> a2h;
     if (QS == S1) {
-        std::vector<float> a2((size_t)d->n_rep * S1 * S1, 0.0f);
+        std::vector<float>& a2 = a2h;
+        a2.assign((size_t)d->n_rep * S1 * S1, 0.0f);
         for (uint32_t ri = 0; ri < d->n_rep; ri++) {
             std::vector<double> acc2((size_t)S1 * S1, 0.0);
             for (uint32_t r = 0; r < d->R; r++) {
@@ -457,23 +507,75 @@ static void build_one_table(DeviceProd* d) {
     d->quiet.alloc(quiet.size());
     CS_CUDA(cudaMemcpy(d->quiet.p, quiet.data(), quiet.size() * 4, cudaMemcpyHostToDevice));
     d->T.quiet = d->quiet.p;
+    // calm_voxel's bound with the largest first-order propensity of a species and the largest pair
+    // propensity (or, without the pair table, the summed second-order rates) for any n particles: one
+    // compare clears most fuller voxels.  Evaluated in binary64 with calm_voxel's margins.
+    std::vector<uint32_t> quiet_n((size_t)d->n_rep * 17, 0u);
+    for (uint32_t ri = 0; ri < d->n_rep; ri++) {
+        double a1 = 0.0, p2 = 0.0;
+        for (uint32_t q = 1; q < S1; q++) a1 = std::max(a1, (double)one[((size_t)ri * S1 + q) * 3]);
+        if (d->T.a2)
+            for (uint32_t i = 0; i < S1 * S1; i++) p2 = std::max(p2, (double)a2h[(size_t)ri * S1 * S1 + i]);
+        else p2 = 2.0 * (double)g23[2 * ri];
+        for (uint32_t n = 3; n < 17; n++) {
+            const double a = n * a1 + 0.5 * n * (n - 1.0) * p2 + n * (n - 1.0) * (n - 2.0) * (double)g23[2 * ri + 1];
+            const double m = std::exp(-a * tau * (1.0 + std::ldexp(1.0, -10))) * 16777216.0 * (1.0 - std::ldexp(1.0, -20));
+            quiet_n[(size_t)ri * 17 + n] = a * tau > 20.0 ? 0u : (uint32_t)std::floor(m);
+        }
+    }
+    d->quiet_n.alloc(quiet_n.size());
+    CS_CUDA(cudaMemcpy(d->quiet_n.p, quiet_n.data(), quiet_n.size() * 4, cudaMemcpyHostToDevice));
+    d->T.quiet_n = d->quiet_n.p;
 }
 
-// Default step before any autotuning: the sweep stream of the model's K with
-// four-block X sweeps and the Y and Z sweeps fused at three blocks per SM
-// (the fastest on the sparse 256^3 lattice measured) where rows have at most
-// 32 words, else four-block sweep passes and a three-block pass 3, else its
-// first brick pass.
-static int pick_default_cfg(uint32_t K, bool fused_ok) {
+static int find_cfg(uint32_t K, int kind, int variant) {
     const auto& c = all_cfgs();
-    int first = -1, plain = -1;
-    for (size_t i = 0; i < c.size(); i++) {
-        if (c[i].K != (int)K) continue;
-        if (c[i].kind == KIND_STREAM && c[i].variant == 4 && fused_ok) return (int)i;
-        if (c[i].kind == KIND_STREAM && c[i].variant == 2) plain = (int)i;
-        if (first < 0 && c[i].kind == KIND_BRICK) first = (int)i;
+    for (size_t i = 0; i < c.size(); i++)
+        if (c[i].K == (int)K && c[i].kind == kind && c[i].variant == variant) return (int)i;
+    throw Error(CS_ERR_LIMIT, "no kernel configuration for this K");
+}
+static uint32_t lists_cap(const DeviceProd* d);
+static uint64_t max_rep_voxels(const DeviceProd* d);
+static bool resident_fits(const DeviceProd* d);
+static bool inplace_fits(const DeviceProd* d);
+static bool fused_fits(const DeviceProd* d);
+
+// Default step before any autotuning (us per frame in runs of 200, and of a call of one frame):
+//  - few particles per replicate (fewer than four replicates: up to 512 at K = 8, 256 at K = 16, as its one block is
+//    then the longer chain; stream / lists, 57 x 47 x 3 with 400 particles 13.4 / 8.6, with 800 14.0 / 13.8
+//    and 41 / 51 in a call of two frames; K = 16, 50^3 with 200 13.4 / 8.4, with 350 13.6 / 12.7 and 39 /
+//    44; 4 replicates of the 12-species network on 30 .. 60 cubed voxels with 400 21.3 / 13.8, 2 replicates 13.9
+//    / 13.8 and 48 / 54): the list form; or, up to 4,608 voxels, the resident form, which needs no
+//    hash but loads the lattice in each call (64 x 64 x 1, 400 particles: resident 5.4 / 14.3, lists 8.3 /
+//    14.1; 109 x 52 x 1, 200 particles: 4.2 / 16.7 against 5.9 / 12.7), up to 1,280 particles
+//    at K = 8, 640 at K = 16 (64 x 64 x 1, K = 16, 1,000 particles, call of two: 52, stream 43);
+//  - up to 2.5 M voxels in all: few or sparse particles the fused sweep stream, whose frame is two dependent
+//    launches against the in-place form's three (stream / in place: 64^3 with 5,000 particles 18.4 / 25.9,
+//    130^3 with 12,000 29.8 / 28.2 and 75 / 77 in a call of two frames, 170^3 with 3,000 30.1 / 24.0; two
+//    fifths of a particle per voxel at most: 20 x 17 x 24 with half of one 34.8 / 25.5).  With one region:
+//    up to 14,336 particles, or one in ten voxels (the 12-species network: 64^3 with 12,000 23.9 / 32.0, with
+//    28,000 38.7 / 35.2, 80^3 with 30,000 33.3 / 36.1, with 60,000 56.9 / 40.2).  Several regions gather
+//    particles in some, and the fullest group sets a pass's time: up to 6,144, or one in 24 voxels (100^3 with
+//    32,000 33.7 / 32.8, 61 x 97 x 45 with 16,000 46.6 / 34.2);
+//  - else the in-place sweep stream;
+//  - rows or edges too long for that: the fused sweep stream at three blocks per SM, or four-block sweep
+//    passes and a three-block pass 3.
+static constexpr uint64_t RESIDENT_DEFAULT_VOXELS = 4608;
+static constexpr uint64_t STREAM_DEFAULT_VOXELS = 2500000;
+static int pick_default_cfg(const DeviceProd* d, bool lists) {
+    if (lists && lists_cap(d)) {
+        const bool small = d->n_rep <= (uint32_t)d->num_sms && max_rep_voxels(d) <= RESIDENT_DEFAULT_VOXELS;
+        if (small && d->p_max * d->K <= 10240u && resident_fits(d)) return find_cfg(d->K, KIND_RESIDENT, 0);
+        if (d->n_rep >= 4u || d->p_max * d->K <= 4096u) return find_cfg(d->K, KIND_LISTS, 0);
     }
-    return plain >= 0 ? plain : first;
+    const int stream = find_cfg(d->K, KIND_STREAM, fused_fits(d) ? 4 : 2);
+    if (!inplace_fits(d)) return stream;
+    if (d->total_voxels <= STREAM_DEFAULT_VOXELS) {
+        const uint64_t V = d->total_voxels, p = d->p_max * d->n_rep;
+        const bool one = d->NC <= 2u;  // one region code beside the outside's
+        if ((p <= (one ? 14336u : 6144u) && 5 * p <= 2 * V) || (one ? 10 : 24) * p <= V) return stream;
+    }
+    return find_cfg(d->K, KIND_INPLACE, 0);
 }
 
 // The region code shared by every lattice voxel of brick w's region window
@@ -501,6 +603,9 @@ static uint32_t window_code(const DeviceProd* d, const RepDesc& r, const WorkIte
 // configuration uses segments of BX planes, x fastest, so that bricks sharing
 // halo planes run close together in time and the halo re-reads hit L2.
 static void build_groups(DeviceProd* d);
+static void build_units(DeviceProd* d);
+static void build_lists(DeviceProd* d);
+static void ensure_slots(DeviceProd* d);
 
 // The fused Y and Z sweeps need every group to hold whole rows.
 static bool fused_fits(const DeviceProd* d) {
@@ -512,6 +617,14 @@ static bool fused_fits(const DeviceProd* d) {
 static void build_items(DeviceProd* d) {
     const KernelCfg& cfg = all_cfgs()[d->cfg_index];
     if (cfg.kind == KIND_RESIDENT) return;  // no work lists: one block per replicate
+    if (cfg.kind == KIND_INPLACE) {
+        build_units(d);
+        return;
+    }
+    if (cfg.kind == KIND_LISTS) {
+        build_lists(d);
+        return;
+    }
     if (cfg.kind == KIND_STREAM) {
         build_groups(d);
         return;
@@ -561,6 +674,14 @@ static void build_items(DeviceProd* d) {
     CS_CUDA(cudaMemcpy(d->items_rep.p, per_rep.data(), per_rep.size() * sizeof(WorkItem), cudaMemcpyHostToDevice));
 }
 
+// Region windows of the bitmap words (wcode, uni); single lattices only.
+static void ensure_wcode(DeviceProd* d) {
+    if (d->h_region_pad.empty() || d->wcode.n != 0) return;
+    d->wcode.alloc(d->occ_words);
+    d->uni.alloc(d->occ_words);
+    region_windows(d->region_pad.p, d->h_reps[0], d->wcode.p, d->uni.p, d->stream);
+}
+
 // Word groups of the sweep stream: for each replicate and x plane, runs of
 // whole rows that fill up to 32 lanes (rows of more than 32 words are cut
 // into 32-word pieces), in replicate order.  The records of group g start
@@ -597,39 +718,7 @@ static void build_groups(DeviceProd* d) {
         throw Error(CS_ERR_LIMIT, "lattice too large for the sweep-stream step (at most 2^32 records)");
     d->n_groups = (uint32_t)gs.size();
     d->n_items = d->n_groups;
-    if (!d->h_region_pad.empty() && d->wcode.n == 0) {
-        // uniform region code of each word's window: first per row word (z from 32k-1 to
-        // 32k+32 inside the lattice), then over the 3 x 3 rows around it
-        const RepDesc& r = d->h_reps[0];
-        const uint64_t rows = (uint64_t)r.X * r.Y;
-        std::vector<uint8_t> run(rows * r.Wz, 0), wc(rows * r.Wz, 0);
-        for (uint64_t row = 0; row < rows; row++) {
-            const uint8_t* rp = d->h_region_pad.data() + row * r.Zr + 2;  // column z + 2 holds z
-            for (uint32_t k = 0; k < r.Wz; k++) {
-                const int64_t za = std::max<int64_t>(0, 32 * (int64_t)k - 1);
-                const int64_t zb = std::min<int64_t>(r.Z, 32 * (int64_t)k + 33);
-                uint8_t c = rp[za];
-                for (int64_t z = za + 1; z < zb && c; z++)
-                    if (rp[z] != c) c = 0;
-                run[row * r.Wz + k] = c;
-            }
-        }
-        for (uint32_t x = 0; x < r.X; x++)
-            for (uint32_t y = 0; y < r.Y; y++)
-                for (uint32_t k = 0; k < r.Wz; k++) {
-                    const uint64_t wi = ((uint64_t)x * r.Y + y) * r.Wz + k;
-                    uint8_t c = run[wi];
-                    for (int dx = -1; dx <= 1 && c; dx++)
-                        for (int dy = -1; dy <= 1 && c; dy++) {
-                            const int64_t xx = (int64_t)x + dx, yy = (int64_t)y + dy;
-                            if (xx < 0 || xx >= r.X || yy < 0 || yy >= r.Y) continue;
-                            if (run[((uint64_t)xx * r.Y + (uint64_t)yy) * r.Wz + k] != c) c = 0;
-                        }
-                    wc[wi] = c;
-                }
-        d->wcode.alloc(wc.size());
-        CS_CUDA(cudaMemcpy(d->wcode.p, wc.data(), wc.size(), cudaMemcpyHostToDevice));
-    }
+    ensure_wcode(d);
     d->groups.alloc(gs.size());
     CS_CUDA(cudaMemcpy(d->groups.p, gs.data(), gs.size() * sizeof(WordGroup), cudaMemcpyHostToDevice));
     d->h_groups = std::move(gs);
@@ -645,6 +734,69 @@ static void build_groups(DeviceProd* d) {
         const uint64_t need = std::max<uint64_t>(1, blocks) * 8ull * STREAM_SSA_OVER_PER_WARP;
         if (d->ssa_over.n < need) d->ssa_over.alloc(need);
     }
+}
+
+// The in-place form needs every edge within a unit's line.
+static bool inplace_fits(const DeviceProd* d) {
+    for (const RepDesc& r : d->h_reps)
+        if (r.X > INPLACE_MAX_EDGE || r.Y > INPLACE_MAX_EDGE || r.Z > INPLACE_MAX_EDGE) return false;
+    return true;
+}
+
+// Units of the in-place form's launches.  An X or Y unit takes whole lines of 2^lw word columns, a Z
+// unit whole rows; each is as large as its block can list (INPLACE_LINE_WORDS, INPLACE_ROW_WORDS)
+// while the launch still has several blocks for every SM.
+static void build_units(DeviceProd* d) {
+    std::vector<LineUnit> u[3];
+    for (int a = 0; a < 3; a++) {
+        d->unit_off[a].assign(d->n_rep + 1, 0);
+        d->unit_words[a] = 1;
+    }
+    const uint64_t line_target = std::min<uint64_t>(INPLACE_LINE_WORDS, d->occ_words / ((uint64_t)d->num_sms * 3));
+    const uint64_t row_target = std::min<uint64_t>(INPLACE_ROW_WORDS, d->occ_words / ((uint64_t)d->num_sms * 6) + 1);
+    for (uint32_t ri = 0; ri < d->n_rep; ri++) {
+        const RepDesc& r = d->h_reps[ri];
+        for (int a = 0; a < 3; a++) d->unit_off[a][ri] = (uint32_t)u[a].size();
+        for (int a = 0; a < 2; a++) {
+            const uint32_t len = a == 0 ? r.X : r.Y, cols = a == 0 ? r.Y * r.Wz : r.Wz;
+            uint32_t lw = 0;
+            while ((1u << lw) < cols && ((uint64_t)len << (lw + 1)) <= line_target) lw++;
+            d->unit_words[a] = std::max(d->unit_words[a], len << lw);
+            for (uint32_t l = 0; l < (a == 0 ? 1u : r.X); l++)
+                for (uint32_t c = 0; c < cols; c += 1u << lw) {
+                    LineUnit w{};
+                    w.rep = ri;
+                    w.a = a == 0 ? c : l;
+                    w.b = (uint16_t)(a == 0 ? 0u : c);
+                    w.n = (uint16_t)std::min(1u << lw, cols - c);
+                    w.lw = (uint16_t)lw;
+                    u[a].push_back(w);
+                }
+        }
+        const uint32_t rows = r.X * r.Y, per = std::max<uint32_t>(1, (uint32_t)(row_target / r.Wz));
+        d->unit_words[2] = std::max(d->unit_words[2], std::min(per, rows) * r.Wz);
+        for (uint32_t row = 0; row < rows; row += per) {
+            LineUnit w{};
+            w.rep = ri;
+            w.a = row;
+            w.n = (uint16_t)std::min(per, rows - row);
+            u[2].push_back(w);
+        }
+    }
+    for (int a = 0; a < 3; a++) {
+        if (u[a].size() > 0x7FFFFFFFull) throw Error(CS_ERR_LIMIT, "lattice too large for the in-place step");
+        d->unit_off[a][d->n_rep] = (uint32_t)u[a].size();
+        d->units[a].alloc(u[a].size());
+        CS_CUDA(cudaMemcpy(d->units[a].p, u[a].data(), u[a].size() * sizeof(LineUnit), cudaMemcpyHostToDevice));
+        if (d->mv[a].n < d->occ_words) d->mv[a].alloc(d->occ_words);
+        if (d->dec[a].n < d->total_voxels) d->dec[a].alloc(d->total_voxels);
+    }
+    if (d->mul.n < d->occ_words) d->mul.alloc(d->occ_words);
+    if (d->spec.n < 32 * d->occ_words) d->spec.alloc(32 * d->occ_words);
+    if (d->react.n < d->occ_words) d->react.alloc(d->occ_words);
+    d->n_items = (uint32_t)u[2].size();
+    d->ip_valid = false;
+    ensure_wcode(d);
 }
 
 // Deals each replicate's word groups heaviest first (most occupied voxels in
@@ -737,6 +889,39 @@ static bool resident_fits(const DeviceProd* d) {
     return v <= 0xFFFFull && resident_smem((int)d->K, v, thr_words(d)) <= (size_t)optin;  // 16-bit voxel lists
 }
 
+// Entries per replicate of the list form for lists of up to p_max particles, or 0 when it does not fit:
+// edges and 10-bit coordinates, reactions only in occupied voxels, and room for three entries per
+// particle (a frame's moves leave about 1.9 entries per particle where a third of the particles move in
+// each sweep), two and a half at least, in one block's shared memory.
+static uint32_t lists_cap(const DeviceProd* d) {
+    if (d->reservoir.n || d->T.n_zero_order) return 0u;
+    for (const RepDesc& r : d->h_reps)
+        if (r.X > LIST_MAX_EDGE || r.Y > LIST_MAX_EDGE || r.Z > LIST_MAX_EDGE) return 0u;
+    int optin = 0;
+    CS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
+    uint32_t lo = 0, hi = 16384;  // the largest capacity that fits
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) / 2u;
+        (lists_smem((int)d->K, mid, thr_words(d)) <= (size_t)optin ? lo : hi) = mid;
+    }
+    if (lo < 64u || d->p_max * 5u > 2ull * lo) return 0u;
+    return (uint32_t)std::min<uint64_t>(lo, std::max<uint64_t>(704, 3 * d->p_max + 64));
+}
+
+static void build_lists(DeviceProd* d) {
+    if (d->ls_state) ensure_slots(d);  // the lists are laid out anew
+    d->ls_state = false;
+    d->l_cap = lists_cap(d);
+    if (d->l_cap == 0u) throw Error(CS_ERR_INVALID_ARG, "list variant needs few particles per replicate (see cs_tiling_kind)");
+    const size_t n = (size_t)d->n_rep * d->l_cap;
+    if (d->l_xyz.n < n) d->l_xyz.alloc(n);
+    if (d->l_cont.n < n * d->K) d->l_cont.alloc(n * d->K);
+    if (d->l_n.n < d->n_rep) d->l_n.alloc(d->n_rep);
+    if (!d->h_flag) CS_CUDA(cudaHostAlloc(&d->h_flag, 4, cudaHostAllocMapped));
+    *d->h_flag = 0u;
+    d->n_items = d->n_rep;
+}
+
 static size_t cfg_smem(const DeviceProd* d, const KernelCfg& cfg) {
     if (cfg.kind == KIND_RESIDENT) return resident_smem(cfg.K, max_rep_voxels(d), thr_words(d));
     if (cfg.kind == KIND_STREAM) return stream_pass_smem(cfg.variant, 2, d->S1, thr_words(d));  // the largest pass
@@ -746,6 +931,14 @@ static size_t cfg_smem(const DeviceProd* d, const KernelCfg& cfg) {
 static void set_attrs(const DeviceProd* d, const KernelCfg& cfg) {
     if (cfg.kind == KIND_RESIDENT) {
         resident_set_attrs(d->device);
+        return;
+    }
+    if (cfg.kind == KIND_INPLACE) {
+        inplace_set_attrs();
+        return;
+    }
+    if (cfg.kind == KIND_LISTS) {
+        lists_set_attrs(d->device);
         return;
     }
     if (cfg.kind == KIND_STREAM) {
@@ -767,6 +960,11 @@ static void drop_graphs(DeviceProd* d) {
             cudaGraphExecDestroy(g1);
             g1 = nullptr;
         }
+    for (cudaGraphExec_t& g1 : d->ip_graph)
+        if (g1) {
+            cudaGraphExecDestroy(g1);
+            g1 = nullptr;
+        }
 }
 
 static void set_cfg(DeviceProd* d, int idx) {
@@ -775,6 +973,12 @@ static void set_cfg(DeviceProd* d, int idx) {
         throw Error(CS_ERR_INVALID_ARG, "fused sweep-stream variant needs rows of at most 32 bitmap words (Z <= 1024)");
     if (cfg.kind == KIND_RESIDENT && !resident_fits(d))
         throw Error(CS_ERR_INVALID_ARG, "resident variant needs every lattice in one block's shared memory");
+    if (cfg.kind == KIND_INPLACE && !inplace_fits(d))
+        throw Error(CS_ERR_INVALID_ARG, "the in-place sweep stream needs edges of at most 1024 voxels");
+    if (cfg.kind == KIND_LISTS && lists_cap(d) == 0u)
+        throw Error(CS_ERR_INVALID_ARG,
+                    "list variant needs few particles per replicate, edges of at most 1024 voxels and no "
+                    "reservoirs or reactions without reactants");
     set_attrs(d, cfg);
     if (cfg.spill >= 0) set_attrs(d, all_cfgs()[cfg.spill]);
     // build_items reads cfg_index; when it refuses the new configuration (a lattice too large for
@@ -1135,9 +1339,6 @@ static DeviceProd* prod_alloc(const Model& m, int device, const std::vector<RepD
     CS_CUDA(cudaMemset(d->counters.p, 0, d->counters.bytes()));
     CS_CUDA(cudaMemset(d->stepbuf.p, 0, 8));
     CS_CUDA(cudaMemset(d->counts.p, 0, d->counts.bytes()));
-    int ci = pick_default_cfg(d->K, fused_fits(d.get()));
-    if (ci < 0) throw Error(CS_ERR_LIMIT, "no kernel configuration for this K");
-    set_cfg(d.get(), ci);
     return d.release();
 }
 
@@ -1158,24 +1359,32 @@ DeviceProd* prod_create(const Model& m, int device) {
     // 16-byte boundary: z is stored at column z + 2 of a row of Zr bytes
     const uint64_t XY = (uint64_t)m.res[0] * m.res[1];
     std::vector<uint8_t> rc(XY * r.Zr, 0);
-    bool any_res = false;
+    bool any_res = false, one_code = true;
     for (uint64_t row = 0; row < XY; row++)
         for (uint32_t z = 0; z < m.res[2]; z++) {
             uint64_t v = row * m.res[2] + z;
             rc[row * r.Zr + z + 2] = (uint8_t)(m.regions[v] + 1);
             any_res |= m.reservoir[v] != 0;
+            one_code &= m.regions[v] == m.regions[0];
         }
     d->region_pad.alloc(rc.size());
     CS_CUDA(cudaMemcpy(d->region_pad.p, rc.data(), rc.size(), cudaMemcpyHostToDevice));
     d->h_region_pad = std::move(rc);
-    build_items(d.get());  // brick items carry their window's region code
+    d->one_code = one_code ? m.regions[0] + 1u : 0u;
     if (any_res) {
         std::vector<uint8_t> r8(m.V);
         for (uint64_t v = 0; v < m.V; v++) r8[v] = (uint8_t)m.reservoir[v];
         d->reservoir.alloc(m.V);
         CS_CUDA(cudaMemcpy(d->reservoir.p, r8.data(), m.V, cudaMemcpyHostToDevice));
+        std::vector<uint32_t> rb(d->occ_words, 0u);
+        for (uint64_t row = 0; row < XY; row++)
+            for (uint32_t z = 0; z < m.res[2]; z++)
+                if (r8[row * m.res[2] + z]) rb[row * d->h_reps[0].Wz + z / 32] |= 1u << (z & 31u);
+        d->resv_bits.alloc(rb.size());
+        CS_CUDA(cudaMemcpy(d->resv_bits.p, rb.data(), rb.size() * 4, cudaMemcpyHostToDevice));
     }
     prod_set_lattice(d.get(), m, m.slots.data());
+    set_cfg(d.get(), pick_default_cfg(d.get(), true));
     return d.release();
 }
 
@@ -1205,6 +1414,9 @@ void prod_set_lattice(DeviceProd* d, const Model& m, const uint32_t* slots) {
     CS_CUDA(cudaStreamSynchronize(d->stream));
     d->cur = 0;
     d->frame_known = false;
+    d->ip_state = d->ip_valid = d->ls_state = d->slots_stale = false;
+    d->p_max = 0;
+    for (uint32_t s = 1; s < d->S1; s++) d->p_max += (uint64_t)cnt[s];
     // the next frame has parity 0 whatever the last one had: its work counters start at zero
     CS_CUDA(cudaMemset(d->counters.p, 0, d->counters.bytes()));
     CS_CUDA(cudaMemcpy(d->slots[0].p, s8.data(), s8.size(), cudaMemcpyHostToDevice));
@@ -1216,6 +1428,7 @@ void prod_set_lattice(DeviceProd* d, const Model& m, const uint32_t* slots) {
 
 void prod_get_lattice(DeviceProd* d, const Model& m, uint32_t* slots, uint32_t* occ, int32_t* conc) {
     DeviceGuard g(d->device);
+    ensure_slots(d);
     CS_CUDA(cudaStreamSynchronize(d->stream));
     uint64_t V = m.V;
     std::vector<uint8_t> s8(V * d->K);
@@ -1291,10 +1504,183 @@ static void launch_resident(DeviceProd* d, uint32_t n, bool batched) {
     }
 }
 
+// Launch parameters of the in-place form but for the units and the frame.
+static InplaceParams inplace_params(const DeviceProd* d) {
+    InplaceParams P{};
+    P.T = d->T;
+    P.reps = d->reps.p;
+    P.lat = d->slots[d->cur].p;
+    P.spec = d->spec.p;
+    P.snap = d->slots[d->cur ^ 1].p;
+    P.occ = d->occ[d->cur].p;
+    P.mul = d->mul.p;
+    P.n_rep = d->n_rep;
+    for (int a = 0; a < 3; a++) {
+        P.mv[a] = d->mv[a].p;
+        P.dec[a] = d->dec[a].p;
+    }
+    P.react = d->react.p;
+    P.resv_bits = d->resv_bits.n ? d->resv_bits.p : nullptr;
+    P.reservoir = d->reservoir.n ? d->reservoir.p : nullptr;
+    P.region_pad = d->region_pad.p;
+    P.wcode = d->wcode.n ? d->wcode.p : nullptr;
+    P.uni = d->uni.n ? d->uni.p : nullptr;
+    P.counts = d->counts.p;
+    P.diag = d->diag.p;
+    P.fa = d->stepbuf.p + d->cur;
+    P.fb = d->stepbuf.p + (d->cur ^ 1);
+    P.thr_smem = thr_words(d) != 0u;
+    return P;
+}
+
+static ListParams lists_params(const DeviceProd* d) {
+    ListParams P{};
+    P.T = d->T;
+    P.reps = d->reps.p;
+    P.lat = d->slots[d->cur].p;
+    P.lat2 = d->slots[d->cur ^ 1].p;
+    P.region_pad = d->region_pad.p;
+    P.code = d->one_code;
+    P.xyz = d->l_xyz.p;
+    P.cont = d->l_cont.p;
+    P.n = d->l_n.p;
+    P.cap = d->l_cap;
+    P.counts = d->counts.p;
+    P.diag = d->diag.p;
+    P.step_out = d->stepbuf.p + d->cur;
+    P.host_flag = d->h_flag;
+    P.thr_words = thr_words(d);
+    return P;
+}
+
+// Writes slots[cur] from the in-place form's or the list form's own layout, for readers of the slots.
+static void ensure_slots(DeviceProd* d) {
+    if (!d->slots_stale) return;
+    if (d->ls_state) lists_unpack((int)d->K, lists_params(d), d->n_rep, max_rep_voxels(d), d->stream);
+    else inplace_unpack((int)d->K, inplace_params(d), d->stream);
+    d->slots_stale = false;
+}
+
+// One launch of the in-place form (axis 0, 1: X and Y sweeps, 2: Z sweep, reactions and the next
+// frame's decisions) over all replicates or over replicate rep.
+static void launch_inplace(DeviceProd* d, int axis, int rep, bool decide_only, bool explicit_frame, uint32_t frame) {
+    InplaceParams P = inplace_params(d);
+    const uint32_t off = rep < 0 ? 0u : d->unit_off[axis][rep];
+    const uint32_t end = rep < 0 ? d->unit_off[axis][d->n_rep] : d->unit_off[axis][rep + 1];
+    P.units = d->units[axis].p + off;
+    P.explicit_frame = explicit_frame ? 1u : 0u;
+    P.frame = frame;
+    P.decide_only = decide_only ? 1u : 0u;
+    inplace_launch((int)d->K, axis, end - off, d->unit_words[axis], d->stream, P);
+}
+
+// n frames of the in-place form.  Batched frames replay captured graphs of kInplaceGraphFrames frames, and
+// one of the frames that remain: a chain of one-frame graphs has a gap of some 4 us at every seam.  The
+// frame number advances on the device.
+static constexpr uint32_t kInplaceGraphFrames = 8;
+
+static void run_inplace(DeviceProd* d, uint32_t n, bool batched) {
+    const bool decided = d->ip_valid && d->ip_frame == d->next_frame && d->ip_epoch == d->seed_epoch;
+    if (!decided) {
+        if (!d->ip_state) {
+            ensure_slots(d);
+            inplace_pack((int)d->K, inplace_params(d), d->stream);
+        }
+        for (auto& m : d->mv) CS_CUDA(cudaMemsetAsync(m.p, 0, m.bytes(), d->stream));
+        CS_CUDA(cudaMemsetAsync(d->react.p, 0, d->react.bytes(), d->stream));
+        launch_inplace(d, 2, -1, true, false, 0u);
+    }
+    // the other buffer takes snapshots from here on, and the lattice is in this form's layout
+    d->occ_valid = false;
+    d->xdec_valid = false;
+    d->ip_valid = false;
+    d->ip_state = true;
+    d->ls_state = false;
+    d->slots_stale = true;
+    if (batched) {
+        auto replay = [&](uint32_t frames) {
+            const uint32_t which = frames - 1u;
+            if (!d->ip_graph[which] || d->ip_graph_cur[which] != d->cur) {
+                if (d->ip_graph[which]) {
+                    cudaGraphExecDestroy(d->ip_graph[which]);
+                    d->ip_graph[which] = nullptr;
+                }
+                cudaGraph_t g;
+                CS_CUDA(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal));
+                for (uint32_t k = 0; k < frames; k++)
+                    for (int axis = 0; axis < 3; axis++) launch_inplace(d, axis, -1, false, false, 0u);
+                CS_CUDA(cudaStreamEndCapture(d->stream, &g));
+                CS_CUDA(cudaGraphInstantiate(&d->ip_graph[which], g, 0));
+                cudaGraphDestroy(g);
+                d->ip_graph_cur[which] = d->cur;
+            }
+            CS_CUDA(cudaGraphLaunch(d->ip_graph[which], d->stream));
+        };
+        uint32_t k = 0;
+        for (; n - k >= kInplaceGraphFrames; k += kInplaceGraphFrames) replay(kInplaceGraphFrames);
+        if (k < n) replay(n - k);
+    } else {
+        for (uint32_t k = 0; k < n; k++)
+            for (uint32_t r = 0; r < d->n_rep; r++)
+                for (int axis = 0; axis < 3; axis++)
+                    launch_inplace(d, axis, (int)r, false, true, (uint32_t)(d->next_frame + k));
+        d->frame_known = false;  // the device's own frame number stayed behind
+    }
+    d->next_frame += n;
+    d->ip_valid = true;
+    d->ip_frame = d->next_frame;
+    d->ip_epoch = d->seed_epoch;
+}
+
+// n frames of the list form; false when the particles have outgrown it (nothing is enqueued then).
+static bool run_lists(DeviceProd* d, uint32_t n, bool batched) {
+    if (*static_cast<volatile uint32_t*>(d->h_flag)) return false;
+    if (d->p_max * 9u > 4ull * d->l_cap) {  // less than 2.25 entries per particle: larger lists, or none
+        const uint32_t cap = lists_cap(d);
+        if (cap <= d->l_cap) return false;
+        build_lists(d);
+    }
+    if (!d->ls_state) {
+        ensure_slots(d);
+        lists_pack((int)d->K, lists_params(d), d->n_rep, max_rep_voxels(d), d->stream);
+    }
+    ListParams P = lists_params(d);
+    P.frame0 = (uint32_t)d->next_frame;
+    P.n_frames = n;
+    // 512 threads where SMs have at most one block anyway: fewer rounds of a sweep's entries
+    const int threads = d->n_rep <= (uint32_t)d->num_sms && d->p_max > 128 ? 512 : 256;
+    if (batched) {
+        lists_launch((int)d->K, threads, P, d->n_rep, d->stream);
+    } else {
+        for (uint32_t r = 0; r < d->n_rep; r++) {
+            P.rep0 = r;
+            lists_launch((int)d->K, threads, P, 1, d->stream);
+        }
+    }
+    d->next_frame += n;
+    d->occ_valid = false;
+    d->xdec_valid = false;
+    d->ip_state = d->ip_valid = false;
+    d->ls_state = true;
+    d->slots_stale = true;
+    return true;
+}
+
 // Enqueues n frames; the frame number must already be in stepbuf[cur] (and
 // its host copy in next_frame).
 static void run_frames_nosync(DeviceProd* d, uint32_t n, bool batched) {
     if (n == 0) return;
+    if (all_cfgs()[d->cfg_index].kind == KIND_LISTS) {
+        if (run_lists(d, n, batched)) return;
+        CS_CUDA(cudaStreamSynchronize(d->stream));
+        set_cfg(d, pick_default_cfg(d, false));
+    }
+    if (all_cfgs()[d->cfg_index].kind == KIND_INPLACE) {
+        run_inplace(d, n, batched);
+        return;
+    }
+    ensure_slots(d);
+    d->ip_state = d->ip_valid = d->ls_state = false;
     if (all_cfgs()[d->cfg_index].kind == KIND_RESIDENT) {
         launch_resident(d, n, batched);
         d->cur ^= (int)(n & 1u);
@@ -1450,6 +1836,12 @@ void prod_get_counts(DeviceProd* d, int64_t* counts) {
     CS_CUDA(cudaStreamSynchronize(d->stream));
     if (d->h_counts[n]) throw Error(CS_ERR_CUDA, kWaitFault);
     for (size_t i = 0; i < n; i++) counts[i] = (int64_t)d->h_counts[i];
+    d->p_max = 0;
+    for (size_t r = 0; r < d->n_rep; r++) {
+        uint64_t p = 0;
+        for (uint32_t s = 1; s < d->S1; s++) p += d->h_counts[r * d->S1 + s];
+        d->p_max = std::max(d->p_max, p);
+    }
 }
 
 void prod_set_counts(DeviceProd* d, const int64_t* counts) {
@@ -1471,6 +1863,15 @@ void prod_render_view(DeviceProd* d, int32_t view, int32_t slice_axis, uint32_t 
         out_dev = tmp.p;
     }
     const RepDesc& r = d->h_reps[0];
+    if (view == 0 && slice == 0u && d->slots_stale) {
+        // the form's own layout is read: far fewer bytes than writing the slots first
+        if (d->ls_state) lists_view((int)d->K, lists_params(d), r, out_dev, d->stream);
+        else inplace_view((int)d->K, inplace_params(d), r, out_dev, d->stream);
+        if (!out_device) CS_CUDA(cudaMemcpyAsync(out_host, out_dev, V * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
+        CS_CUDA(cudaStreamSynchronize(d->stream));
+        return;
+    }
+    ensure_slots(d);
     ViewParams v{};
     v.slots = d->slots[d->cur].p;
     v.K = d->K;
@@ -1482,7 +1883,8 @@ void prod_render_view(DeviceProd* d, int32_t view, int32_t slice_axis, uint32_t 
     v.slice_axis = slice_axis;
     v.slice = slice;
     v.out = out_dev;
-    render_view_kernel<<<1024, 256, 0, d->stream>>>(v);
+    if (view == 0 && slice == 0u) launch_majority_view(d->K, v.slots, V, out_dev, d->stream);
+    else render_view_kernel<<<1024, 256, 0, d->stream>>>(v);
     CS_LAUNCH_CHECK();
     if (!out_device) CS_CUDA(cudaMemcpyAsync(out_host, out_dev, V * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
     CS_CUDA(cudaStreamSynchronize(d->stream));
@@ -1568,6 +1970,8 @@ DeviceProd* prod_ensemble_create(const Model& m, uint32_t n, const uint32_t* res
     d->occ_valid = false;
     CS_CUDA(cudaMemcpy(d->counts.p, cnt.data(), cnt.size() * 8, cudaMemcpyHostToDevice));
     d->cur = 0;
+    for (uint32_t s = 1; s < d->S1; s++) d->p_max += init_counts[s];
+    set_cfg(d.get(), pick_default_cfg(d.get(), true));
     return d.release();
 }
 
@@ -1591,6 +1995,7 @@ uint32_t prod_s1(const DeviceProd* d) { return d->S1; }
 // Downloads the packed slots of every replicate (K bytes per voxel).
 void prod_get_slots_raw(DeviceProd* d, uint8_t* out) {
     DeviceGuard g(d->device);
+    ensure_slots(d);
     CS_CUDA(cudaStreamSynchronize(d->stream));
     CS_CUDA(cudaMemcpy(out, d->slots[d->cur].p, d->total_voxels * d->K, cudaMemcpyDeviceToHost));
 }
@@ -1622,12 +2027,14 @@ void prod_tiling_desc(int i, int* K, int* TY, int* TZ, int* NT) {
 void prod_tiling_kind(int i, int* kind, int* BX) {
     const auto& c = all_cfgs();
     if (i < 0 || i >= (int)c.size()) throw Error(CS_ERR_INVALID_ARG, "tile configuration index out of range");
-    *kind = c[i].kind; *BX = c[i].BX;
+    *kind = c[i].kind == KIND_INPLACE ? KIND_STREAM : c[i].kind; *BX = c[i].BX;
 }
 int prod_tiling_launches(int i) {
     const auto& c = all_cfgs();
     if (i < 0 || i >= (int)c.size()) throw Error(CS_ERR_INVALID_ARG, "tile configuration index out of range");
     if (c[i].kind == KIND_RESIDENT) return 1;  // one launch per step call
+    if (c[i].kind == KIND_LISTS) return 1;
+    if (c[i].kind == KIND_INPLACE) return 3;
     if (c[i].kind == KIND_STREAM) {
         if (stream_variant_frames(c[i].variant)) return 1;  // one launch per step call
         return stream_variant_fused(c[i].variant) ? 2 : 3;
@@ -1674,11 +2081,14 @@ float prod_time_frames(DeviceProd* d, uint32_t n, uint64_t frame0, bool batched)
 namespace cellsim {
 // Autotuner: times every compiled configuration for this K on the handle's
 // own lattice and keeps the fastest.  Each trial starts from a device copy of
-// the current state and the state is restored afterwards, so tuning does not
-// advance or change the simulation (every configuration computes the same
+// the state 64 frames on (a freshly placed lattice settles first: 60 x 61 x 64
+// with the stiff network took the in-place form, best in its first frames, and
+// then 1,930 us per 51 frames where a brick variant takes 1,700), and the state
+// is restored afterwards, so tuning does not advance or change the simulation (every configuration computes the same
 // frame anyway).  Choices are cached per (K, species, reactions, regions,
 // zero-order reactions or reservoirs present, lattice shapes, device) for the
 // life of the process.
+static constexpr uint32_t kSettleFrames = 64;
 int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched, float* best_ms) {
     DeviceGuard g(d->device);
     static std::mutex mu;
@@ -1688,7 +2098,9 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
     std::string key = std::string(prop.name) + "|" + std::to_string(d->K) + "," + std::to_string(d->S1) + "," +
                       std::to_string(d->R) + "," + std::to_string(d->NC) + "," + std::to_string(batched ? 1 : 0) +
                       // reservoirs and zero-order reactions make the brick pass step every interior voxel
-                      "," + std::to_string(d->T.n_zero_order != 0u ? 1 : 0) + std::to_string(d->reservoir.n ? 1 : 0);
+                      "," + std::to_string(d->T.n_zero_order != 0u ? 1 : 0) + std::to_string(d->reservoir.n ? 1 : 0) +
+                      // whether the particles leave the list form among the candidates
+                      (lists_cap(d) ? "L" : "");
     for (const RepDesc& r : d->h_reps) key += "|" + std::to_string(r.X) + "x" + std::to_string(r.Y) + "x" + std::to_string(r.Z);
     {
         std::lock_guard<std::mutex> lk(mu);
@@ -1706,26 +2118,43 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
     if (frames == 0) frames = 1;
     CS_CUDA(cudaStreamSynchronize(d->stream));
     const size_t bytes = (size_t)d->total_voxels * d->K;
-    DevBuf<uint8_t> keep;
-    keep.alloc(bytes);
-    DevBuf<unsigned long long> keep_counts;
-    keep_counts.alloc(d->counts.n);
-    DevBuf<uint32_t> keep_diag;
-    keep_diag.alloc(PD_N);
+    struct Kept {
+        DevBuf<uint8_t> slots;
+        DevBuf<unsigned long long> counts;
+        DevBuf<uint32_t> diag;
+    } start, settled;
     const int cur0 = d->cur;
-    CS_CUDA(cudaMemcpyAsync(keep.p, d->slots[cur0].p, bytes, cudaMemcpyDeviceToDevice, d->stream));
-    CS_CUDA(cudaMemcpyAsync(keep_counts.p, d->counts.p, d->counts.bytes(), cudaMemcpyDeviceToDevice, d->stream));
-    CS_CUDA(cudaMemcpyAsync(keep_diag.p, d->diag.p, PD_N * 4, cudaMemcpyDeviceToDevice, d->stream));
+    auto save = [&](Kept& k) {
+        k.slots.alloc(bytes);
+        k.counts.alloc(d->counts.n);
+        k.diag.alloc(PD_N);
+        ensure_slots(d);
+        CS_CUDA(cudaMemcpyAsync(k.slots.p, d->slots[d->cur].p, bytes, cudaMemcpyDeviceToDevice, d->stream));
+        CS_CUDA(cudaMemcpyAsync(k.counts.p, d->counts.p, d->counts.bytes(), cudaMemcpyDeviceToDevice, d->stream));
+        CS_CUDA(cudaMemcpyAsync(k.diag.p, d->diag.p, PD_N * 4, cudaMemcpyDeviceToDevice, d->stream));
+    };
+    const Kept* from = &start;
     auto restore = [&]() {
-        CS_CUDA(cudaMemcpyAsync(d->slots[cur0].p, keep.p, bytes, cudaMemcpyDeviceToDevice, d->stream));
-        CS_CUDA(cudaMemcpyAsync(d->counts.p, keep_counts.p, d->counts.bytes(), cudaMemcpyDeviceToDevice, d->stream));
-        CS_CUDA(cudaMemcpyAsync(d->diag.p, keep_diag.p, PD_N * 4, cudaMemcpyDeviceToDevice, d->stream));
+        CS_CUDA(cudaMemcpyAsync(d->slots[cur0].p, from->slots.p, bytes, cudaMemcpyDeviceToDevice, d->stream));
+        CS_CUDA(cudaMemcpyAsync(d->counts.p, from->counts.p, d->counts.bytes(), cudaMemcpyDeviceToDevice, d->stream));
+        CS_CUDA(cudaMemcpyAsync(d->diag.p, from->diag.p, PD_N * 4, cudaMemcpyDeviceToDevice, d->stream));
         CS_CUDA(cudaMemsetAsync(d->counters.p, 0, d->counters.bytes(), d->stream));  // parity cur0 starts afresh
         CS_CUDA(cudaStreamSynchronize(d->stream));
         d->cur = cur0;
         d->occ_valid = false;
+        d->ip_state = d->ip_valid = d->ls_state = d->slots_stale = false;
         d->frame_known = false;
     };
+    save(start);
+    size_t free_bytes = 0, all_bytes = 0;
+    CS_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
+    if (free_bytes > 4 * bytes) {  // else the trials start from the current state
+        prod_time_frames(d, kSettleFrames, frame0, batched);
+        save(settled);
+        frame0 += kSettleFrames;
+        from = &settled;
+        restore();
+    }
     const auto& c = all_cfgs();
     int best = -1;
     float best_t = 0.0f;
@@ -1733,6 +2162,8 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         if (c[i].K != (int)d->K) continue;
         if (c[i].kind == KIND_STREAM && stream_variant_fused(c[i].variant) && !fused_fits(d)) continue;
         if (c[i].kind == KIND_RESIDENT && !resident_fits(d)) continue;
+        if (c[i].kind == KIND_INPLACE && !inplace_fits(d)) continue;
+        if (c[i].kind == KIND_LISTS && !lists_cap(d)) continue;
         d->seg_len = 0;
         set_cfg(d, i);
         prod_time_frames(d, 2, frame0, batched);  // warm-up: graph, bitmaps, caches
@@ -1750,6 +2181,8 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         if (best < 0 || t < best_t) { best = i; best_t = t; }
     }
     set_cfg(d, best);
+    from = &start;
+    restore();
     {
         std::lock_guard<std::mutex> lk(mu);
         cache[key] = {best, best_t};

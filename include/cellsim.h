@@ -288,18 +288,28 @@ cs_status cs_step_philox_timed(cs_sim* sim, uint32_t n_steps, uint64_t seed, flo
  * autotuner.  cs_tiling_kind: kind 0 = tile pipeline over (TY x TZ tile,
  * x-segment) items; kind 1 = sparse brick pass over brick_planes x TY x TZ
  * bricks, crowded bricks finished by a full-capacity second brick pass;
- * kind 2 = sweep stream (the default): barrier-free passes over groups of 32
+ * kind 2 = sweep stream: barrier-free passes over groups of 32
  * occupancy-bitmap words (TZ = 32, brick_planes = 0; TY = 1 marks the
  * persistent form that runs every frame of a step call in one launch, TY = 0
- * the per-pass launches); kind 3 = resident form: one block of `threads`
+ * the per-pass launches), or with TY = 2 its in-place form, which makes every
+ * decision of a frame in one pass and sweeps only the voxels that change
+ * (edges of at most 1024 voxels; the default for lattices the list form does
+ * not take); kind 3 = resident form: one block of `threads`
  * per replicate holds its lattice in shared memory for every frame of a step
  * call (TY = TZ = 0; about 5,300 voxels per replicate at K = 16 and 9,000 at
- * K = 8 at most: cs_set_tiling refuses larger lattices).  Every variant
+ * K = 8 at most: cs_set_tiling refuses larger lattices); kind 4 = list form:
+ * one block per replicate keeps the list of its occupied voxels for every
+ * frame of a step call (up to about 1,000 particles per replicate at K = 16
+ * and 1,300 at K = 8, edges of at most 1024 voxels, no reservoirs and no
+ * reactions without reactants: cs_set_tiling refuses others; a replicate that
+ * outgrows it within a call is finished over its whole lattice, and the first
+ * call made after that has happened on the device takes the in-place form).  A new handle takes the resident
+ * form (small lattices), the list form or the in-place form.  Every variant
  * computes the same lattice.  cs_tiling_launches: kernel launches per frame
  * once a run is under way (the sweep stream: 3, or 2 where the Y and Z sweeps
  * are one launch, or 1 per step call in the persistent form; the last two need
- * Z <= 1024 and cs_set_tiling refuses them otherwise; the resident form: 1
- * per step call).  No reference counterpart (the reference has one
+ * Z <= 1024 and cs_set_tiling refuses them otherwise; the in-place form: 3;
+ * the resident and list forms: 1 per step call).  No reference counterpart (the reference has one
  * fixed dispatch shape per shader). */
 cs_status cs_tiling_count(int32_t* n);
 cs_status cs_tiling_describe(int32_t index, int32_t* K, int32_t* TY, int32_t* TZ, int32_t* threads);
