@@ -13,36 +13,51 @@
 // K for some voxel (`contended`), a one-thread kernel redoes the frame's
 // diffusion in serial order with the capacity rule.
 //
-// cs_step runs the sparse form on single (in-place) state buffers.  Each pass
-// is a grid-stride loop over a voxel list compacted from a bitmap (one atomic
-// per warp, word order kept within a warp), so every lane has a voxel however
-// sparse the lattice.  Six launches per frame:
-//   ref_sp_list_act     the act list: voxels holding a particle, a non-zero
-//                       occupancy or a non-zero species count.
-//   ref_sp_directions   over the act list: the direction of every particle
-//                       from PCG(itime + x%y + z + slot index)
-//                       (rdme.wgsl:138-226); voxels with a departure store
-//                       their directions and a snapshot of their slots and set
-//                       their `dep` bit; every departure counts one arrival at
-//                       its destination, sets both voxels' `touch` bits and
-//                       raises `contended` when the destination could overflow.
-//   ref_sp_list_touch   the touch list and the union of act and touch.
-//   ref_sp_gather       (not contended) over the touch list: the gather above,
-//                       in place, with the species of arriving particles read
-//                       from their sources' snapshots and the concentrations
-//                       updated in place.
-//   ref_sp_serial       (contended) one thread: the serial diffusion, in place.
-//   ref_sp_cme          over the union list: one-event reaction test, rewrite
+// cs_step runs the sparse form on single (in-place) state buffers.  A block
+// takes a range of words of the voxel bitmaps and lists their voxels in shared
+// memory, so every lane has a voxel however sparse the lattice, and no list
+// passes through global memory.  Three launches per frame:
+//   ref_sp_directions   over act (voxels holding a particle, a non-zero
+//                       occupancy or a non-zero species count): the direction
+//                       of every particle from PCG(itime + x%y + z + slot
+//                       index) (rdme.wgsl:138-226); voxels with a departure
+//                       store their directions and a snapshot of their slots
+//                       and set their `dep` bit; every departure counts one
+//                       arrival at its destination, sets both voxels' `touch`
+//                       bits and raises `contended` when the destination could
+//                       overflow.
+//   ref_sp_move         not contended: over touch, the gather above, in place,
+//                       with the species of arriving particles read from their
+//                       sources' snapshots; contended: one thread of one
+//                       block, the serial diffusion, in place.
+//   ref_sp_cme          over act and touch: one-event reaction test, rewrite
 //                       with rollback, stable compaction (final_stage.wgsl:25-33),
 //                       species-count deltas reduced per block; the next
-//                       frame's act bitmap.
-// A voxel on neither list holds no particle and no species count, its slots
+//                       frame's act words.
+// Occupancy and the concentration row (68 bytes at 16 species) of nearly every
+// voxel are what its slots say; such a voxel is `tidy`, and the passes neither
+// read nor write the two for it: they are written when somebody reads them.
+// A voxel stops being tidy when a reaction leaves a count that its slots
+// cannot show (below zero, or skipped for a reservoir species).  A tidy voxel
+// with one particle fires with a probability that depends on the species
+// alone, tabulated by the same operations in the same order; the others sum
+// only reactions whose reactants are all present (the rest add zeros).
+//
+// What bounds it: up to 64 cubed three launch latencies (40 cubed with 3,000
+// particles 15.3 us per frame, 37.2 with six launches, two of them list
+// compactions, and the rows read and written throughout); past that the
+// scattered accesses per listed voxel (100 cubed with 40,000 24.2, before
+// 51.9; 160 cubed with 200,000 47.1, before 84.6).  Calls of 20 frames and a
+// view of 128 cubed with 22,000 particles: 989 -> 424 us; of 10 frames and a
+// view of 256 cubed with 1 M: 2,856 -> 1,657 us.
+//
+// A voxel in neither act nor touch holds no particle and no species count, its slots
 // are compacted and its conc[v][0] is already 1, so the reaction pass leaves
 // it unchanged unless its first uniform is 0: r1 = UniformFloat(PCG(itime +
 // x*y + z)) is 0 exactly when the seed is 0 (PCG and the xorshift are
 // bijections that fix 0), and r1 <= 1 - exp(-0 * tau) = 0 then fires the
-// selection.  Pass 1 puts those voxels (x*y + z = -itime mod 2^32) on the
-// touch list.  The first frame after an upload, and every frame of a model
+// selection.  Pass 1 puts those voxels (x*y + z = -itime mod 2^32) in
+// touch.  The first frame after an upload, and every frame of a model
 // with a reaction without reactants (non-zero propensity in every voxel), run
 // the reaction pass over every voxel.
 //
@@ -53,6 +68,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -93,10 +109,13 @@ struct DeviceRef {
     DevBuf<float> P, rates;
     DevBuf<int32_t> stoich, stat;
     DevBuf<uint32_t> reactants, diag, flag, itimes;
-    DevBuf<uint32_t> act_bm[2], touch_bm, dep_bm, act_list, touch_list, union_list, cnt, arrivals;
+    DevBuf<uint32_t> act_bm, touch_bm, dep_bm, tidy_bm, same_bm, uses, arrivals;
+    DevBuf<float> fire1;
     DevBuf<int32_t> sample_ring;
-    uint32_t par = 0;         // parity of the next frame's lists
-    int grid = 1;             // blocks of the sparse passes (grid-stride loops)
+    int sms = 1, smem_optin = 0;
+    bool finite = true;         // every rate is finite
+    bool one_block = false;     // the frames of a call run in one block (ref_choose_form)
+    bool rows_stale = false;    // frames have run since the tidy voxels' rows were written
     bool dense_next = true;   // the next reaction pass visits every voxel (first frame after an upload)
     bool dense_always = false;  // a reaction without reactants: every voxel may fire in every frame
     ~DeviceRef() {
@@ -468,269 +487,347 @@ __global__ void ref_cme(RefParams p, uint8_t* __restrict__ dst, uint32_t* __rest
 
 // ------------------------------------------------------------------ sparse form
 
-// Bitmaps over the linear voxel index (word i holds voxels 32i .. 32i+31) and
-// the voxel lists compacted from them, for a frame of parity c:
-//   act bitmap c   voxels that hold a particle, a non-zero occupancy or a
-//                  non-zero species count (s >= 1); the reaction pass sets
-//                  act bitmap c ^ 1 for the next frame
-//   touch bitmap   voxels that gain or lose particles this frame, or whose
-//                  reaction seed is 0
-//   dep bitmap     voxels with a departure this frame
-//   act list       act bitmap c, compacted at the start of the frame
-//   touch list     the touch bitmap, compacted after the directions pass
-//   union list     act bitmap c | touch bitmap, compacted with it
-// cnt[0..2]: entries of the act, touch and union lists.
+// Bitmaps over the linear voxel index (word i holds voxels 32i .. 32i+31):
+//   act    voxels that hold a particle, a non-zero occupancy or a non-zero
+//          species count (s >= 1)
+//   touch  voxels that gain or lose particles this frame, or whose reaction
+//          seed is 0
+//   dep    voxels with a departure this frame
+//   tidy   voxels whose occupancy and species counts are those of their slots:
+//          no pass reads or writes the two arrays for them (ref_write_rows
+//          does when somebody asks for them)
+//   same   voxels whose six neighbours lie in the lattice and share their region
+// A block owns ranges of cw consecutive words and lists their voxels in shared
+// memory; no launch keeps a list in global memory.
 struct RefSparse {
-    uint32_t* act_bm[2];
-    uint32_t* touch_bm;
-    uint32_t* dep_bm;
-    uint32_t* act_list;
-    uint32_t* touch_list;
-    uint32_t* union_list;
-    uint32_t* cnt;       // [3]
-    uint32_t* arrivals;  // [V] particles moving into the voxel this frame (zero between frames)
-    uint8_t* dirs;       // [V*K] direction codes of a voxel with a departure (7 = stays)
-    uint8_t* snap;       // [V*K] slots of a voxel with a departure, as the frame started
-    uint32_t W;          // bitmap words
-    uint32_t c;          // frame parity
+    uint32_t* act;
+    uint32_t* touch;
+    uint32_t* dep;
+    uint32_t* tidy;
+    const uint32_t* same;
+    uint32_t* arrivals;    // [V] particles moving into the voxel this frame (zero between frames)
+    uint8_t* dirs;         // [V*K] direction codes of a voxel with a departure (7 = stays)
+    uint8_t* snap;         // [V*K] slots of a voxel with a departure, as the frame started
+    const uint32_t* uses;  // [S1][UW] reactions (bit r) that need species s
+    const float* fire1;    // [S1] firing probability of an empty voxel (0) or of a sole particle of species q
+    uint32_t W;            // bitmap words
+    uint32_t cw;           // words of a range
+    uint32_t UW;           // words of a reaction mask
+    uint32_t finite;       // every rate is finite: a reaction that lacks a reactant adds 0
 };
 
-// act bitmaps of this frame and the next, chosen by select (indexing the kernel parameter's
-// array by a run-time value would copy the parameters to local memory)
-__device__ __forceinline__ uint32_t* act_cur(const RefSparse& sp) { return sp.c ? sp.act_bm[1] : sp.act_bm[0]; }
-__device__ __forceinline__ uint32_t* act_next(const RefSparse& sp) { return sp.c ? sp.act_bm[0] : sp.act_bm[1]; }
-
-__device__ __forceinline__ bool bit_of(const uint32_t* bm, uint32_t v) { return (__ldcg(bm + (v >> 5)) >> (v & 31u)) & 1u; }
+// A word that other blocks or threads write (global memory, or shared memory in the one-block form).
+__device__ __forceinline__ uint32_t ref_word(const uint32_t* p) { return *reinterpret_cast<const volatile uint32_t*>(p); }
+__device__ __forceinline__ bool bit_of(const uint32_t* bm, uint32_t v) { return (ref_word(bm + (v >> 5)) >> (v & 31u)) & 1u; }
 __device__ __forceinline__ void set_bit(uint32_t* bm, uint32_t v) { atomicOr(bm + (v >> 5), 1u << (v & 31u)); }
 
-__device__ __forceinline__ uint32_t grid_threads() { return gridDim.x * blockDim.x; }
-__device__ __forceinline__ uint32_t grid_tid() { return blockIdx.x * blockDim.x + threadIdx.x; }
+// Byte tests on slot registers: bit 7 of byte i of the result is the answer for slot i.
+__device__ __forceinline__ uint64_t bytes_nonzero(uint64_t x) {
+    return (((x & 0x7F7F7F7F7F7F7F7Full) + 0x7F7F7F7F7F7F7F7Full) | x) & 0x8080808080808080ull;
+}
+struct RefMask {
+    uint64_t lo, hi;
+};
+__device__ __forceinline__ RefMask rs_valid(uint32_t K) {  // the K slots
+    const uint64_t b = 0x8080808080808080ull;
+    return RefMask{K >= 8u ? b : b & ((1ull << (8u * K)) - 1ull), K >= 16u ? b : K > 8u ? b & ((1ull << (8u * (K - 8u))) - 1ull) : 0ull};
+}
+__device__ __forceinline__ uint32_t rm_count(const RefMask& m) { return (uint32_t)(__popcll(m.lo) + __popcll(m.hi)); }
+__device__ __forceinline__ bool rm_any(const RefMask& m) { return (m.lo | m.hi) != 0ull; }
+// the lowest marked slot (one must be)
+__device__ __forceinline__ uint32_t rm_first(const RefMask& m) {
+    return m.lo ? (uint32_t)(__ffsll((long long)m.lo) - 1) >> 3 : 8u + ((uint32_t)(__ffsll((long long)m.hi) - 1) >> 3);
+}
+__device__ __forceinline__ void rm_drop(RefMask& m) {
+    if (m.lo) m.lo &= m.lo - 1ull;
+    else m.hi &= m.hi - 1ull;
+}
+__device__ __forceinline__ RefMask rs_full(const RefSlots& a) { return RefMask{bytes_nonzero(a.lo), bytes_nonzero(a.hi)}; }
+__device__ __forceinline__ uint32_t rs_count(const RefSlots& a) { return rm_count(rs_full(a)); }
 
-// Appends the voxels of bitmap word `m` (word index i) to a list, every lane of
-// the warp calling it with its own word: one atomic per warp reserves the
-// warp's entries, which keep word order within the warp.
-__device__ __forceinline__ void warp_compact(uint32_t m, uint32_t i, uint32_t* list, uint32_t* counter) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n = (uint32_t)__popc(m);
+// The library's own buffers: K = KT (16 or 8), vector access; KT = 0: any K.
+template <int KT>
+__device__ __forceinline__ RefSlots rk_load(const uint8_t* base, uint32_t v, uint32_t K) {
+    if constexpr (KT == 16) {
+        const uint4 t = *reinterpret_cast<const uint4*>(base + (size_t)v * 16u);
+        return RefSlots{(uint64_t)t.x | ((uint64_t)t.y << 32), (uint64_t)t.z | ((uint64_t)t.w << 32)};
+    } else if constexpr (KT == 8) {
+        const uint2 t = *reinterpret_cast<const uint2*>(base + (size_t)v * 8u);
+        return RefSlots{(uint64_t)t.x | ((uint64_t)t.y << 32), 0ull};
+    } else {
+        return rs_load(base + (size_t)v * K, K);
+    }
+}
+template <int KT>
+__device__ __forceinline__ void rk_store(uint8_t* base, uint32_t v, uint32_t K, const RefSlots& a) {
+    rs_store(base + (size_t)v * K, KT ? (uint32_t)KT : K, a);
+}
+
+// Programmatic dependent launch between the passes of a frame: a pass lets the next one launch at
+// once, stages the tables that no launch writes, and waits for the previous pass to complete (and
+// its memory to be visible) before it touches anything else; without a programmatic dependency the
+// wait returns at once.
+__device__ __forceinline__ void ref_allow_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void ref_wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// Each pass is a device body, run by its own launch or, on small lattices, by the one-block form
+// ref_sp_frames_block.  Shared memory of a body: the range's word areas and list, then its tables.
+enum : int { RW_A, RW_B, RW_C, REF_AREAS };
+struct RefRange {
+    uint32_t* area[REF_AREAS];  // [cw] each
+    uint16_t* list;             // [32 * cw] (word << 5) | bit
+    uint32_t* tmp;              // [32]
+};
+__host__ __device__ constexpr size_t ref_range_words(uint32_t cw) { return REF_AREAS * (size_t)cw + 16 * (size_t)cw + 32; }
+__device__ __forceinline__ RefRange ref_range(uint32_t* sm, uint32_t cw) {
+    RefRange r;
+    for (int a = 0; a < REF_AREAS; a++) r.area[a] = sm + a * cw;
+    r.list = reinterpret_cast<uint16_t*>(sm + REF_AREAS * cw);
+    r.tmp = sm + (REF_AREAS + 16) * cw;
+    return r;
+}
+
+// Lists the voxels of the range's words (thread t's word m is word t of the range, 0 past the
+// range), in word order; every thread of the block calls it.  Returns how many there are.  The
+// caller's barrier comes before the next call.
+template <int NT>
+__device__ __forceinline__ uint32_t ref_list(uint32_t m, const RefRange& R) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, n = (uint32_t)__popc(m);
     uint32_t incl = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += u;
+        if ((int)lane >= o) incl += u;
     }
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0u) return;
-    uint32_t base = 0;
-    if (lane == 31u) base = atomicAdd(counter, total);
-    base = __shfl_sync(0xffffffffu, base, 31) + incl - n;
-    for (; m; m &= m - 1u) list[base++] = i * 32u + (uint32_t)(__ffs((int)m) - 1);
-}
-
-// Programmatic dependent launch between the passes of a frame: a pass lets the next one launch at
-// once and waits for the previous one to complete (and its memory to be visible) before it touches
-// anything; without a programmatic dependency the wait returns at once.
-__device__ __forceinline__ void ref_pdl_start() {
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-}
-
-// Each pass is a device body with grid-stride loops, run by its own launch (a thin kernel that
-// waits for the previous pass first) or, on small lattices, by the one-block form
-// ref_sp_frames_block.
-
-// The act list of act bitmap c.
-__device__ __forceinline__ void ref_sp_list_act_body(RefSparse sp) {
-    for (uint32_t i0 = grid_tid() & ~31u; i0 < sp.W; i0 += grid_threads()) {
-        const uint32_t i = i0 + (threadIdx.x & 31u);
-        warp_compact(i < sp.W ? act_cur(sp)[i] : 0u, i, sp.act_list, sp.cnt + 0);
+    if (lane == 31u) R.tmp[w] = incl;
+    __syncthreads();
+    uint32_t at = incl - n, total = 0;
+#pragma unroll
+    for (int i = 0; i < NT / 32; i++) {
+        const uint32_t t = R.tmp[i];
+        if (i < (int)w) at += t;
+        total += t;
     }
+    for (; m; m &= m - 1u) R.list[at++] = (uint16_t)((threadIdx.x << 5) | (uint32_t)(__ffs((int)m) - 1));
+    __syncthreads();
+    return total;
 }
 
-__global__ void __launch_bounds__(256) ref_sp_list_act(RefSparse sp) {
-    ref_pdl_start();
-    ref_sp_list_act_body(sp);
-}
-
-// The touch list, and the union list of act bitmap c and the touch bitmap.
-__device__ __forceinline__ void ref_sp_list_touch_body(RefSparse sp) {
-    for (uint32_t i0 = grid_tid() & ~31u; i0 < sp.W; i0 += grid_threads()) {
-        const uint32_t i = i0 + (threadIdx.x & 31u);
-        const uint32_t t = i < sp.W ? __ldcg(sp.touch_bm + i) : 0u;
-        const uint32_t a = i < sp.W ? act_cur(sp)[i] : 0u;
-        warp_compact(t, i, sp.touch_list, sp.cnt + 1);
-        warp_compact(a | t, i, sp.union_list, sp.cnt + 2);
-    }
-}
-
-__global__ void __launch_bounds__(256) ref_sp_list_touch(RefSparse sp) {
-    ref_pdl_start();
-    ref_sp_list_touch_body(sp);
-}
-
-// Pass 1: directions of every particle of the act list; departures, arrival
-// counts, touched voxels and the contention test.  Also marks the voxels whose
-// reaction seed itime + x*y + z is 0 this frame, clears act bitmap c ^ 1 (the
-// reaction pass fills it) and the touch and union list counters.
-__device__ __forceinline__ void ref_sp_directions_body(RefParams p, RefSparse sp, const uint8_t* slots,
-                                                       const uint32_t* occ, const uint32_t* itimes, uint32_t step,
-                                                       uint32_t* diag, uint32_t* contended, uint32_t stage_P) {
-    const uint32_t itime = __ldg(itimes + step);
-    const uint32_t K = p.K;
-    const uint32_t n = __ldcg(sp.cnt + 0);
-    if (grid_tid() == 0) {
-        sp.cnt[1] = 0u;
-        sp.cnt[2] = 0u;
-    }
-    // the probability table in shared memory when the launch gave room for it
-    extern __shared__ float s_P[];
-    const float* Pt = p.P;
-    if (stage_P) {
+__device__ __forceinline__ void ref_stage_P(const RefParams& p, float* s_P, uint32_t stage_P) {
+    if (stage_P)
         for (uint32_t i = threadIdx.x; i < p.NR * p.NR * p.S1; i += blockDim.x) s_P[i] = p.P[i];
-        __syncthreads();
-        Pt = s_P;
-    }
-    for (uint32_t i = grid_tid(); i < sp.W; i += grid_threads()) act_next(sp)[i] = 0u;
-    const uint32_t XY = p.X * p.Y;
-    for (uint32_t g = grid_tid(); g < XY; g += grid_threads()) {
-        const uint32_t x = g / p.Y, y = g - x * p.Y;
-        const uint32_t z = 0u - itime - x * y;  // u32 wrap, as the shader's seed arithmetic
-        if (z < p.Z) set_bit(sp.touch_bm, g * p.Z + z);
-    }
-    for (uint32_t e = grid_tid(); e < n; e += grid_threads()) {
-        const uint32_t v = sp.act_list[e];
-        uint32_t o = occ[v];
-        if (o > K) {
-            // the gather's contention test fails for this voxel whatever arrives
-            atomicAdd(diag + DIAG_OCC_RANGE, 1u);
-            atomicOr(contended, 1u);
-            o = K;
-        }
-        const RefSlots sl = rs_load(slots + (size_t)v * K, K);
-        uint32_t x, y, z;
-        ref_coords(p, v, x, y, z);
-        const uint8_t* reg = p.regions;
-        uint32_t rn[7] = {reg[v], 0u, 0u, 0u, 0u, 0u, 0u};
-        if (x > 0u) rn[1] = reg[v - p.YZ];
-        if (x < p.X - 1u) rn[2] = reg[v + p.YZ];
-        if (y > 0u) rn[3] = reg[v - p.Z];
-        if (y < p.Y - 1u) rn[4] = reg[v + p.Z];
-        if (z > 0u) rn[5] = reg[v - 1];
-        if (z < p.Z - 1u) rn[6] = reg[v + 1];
-        bool has_dep = false;
-        RefSlots dr{0x0707070707070707ull, 0x0707070707070707ull};  // 7: stays
-        for (uint32_t s = 0; s < K; s++) {
-            const uint32_t q = rs_get(sl, s);
-            if (s < o && q != 0u) {
-                const int d = ref_decide_rn(p, Pt, rn, x, y, z, q, v * K + s, itime);
-                rs_set(dr, s, (uint32_t)d);
-                has_dep |= d < 6;
+}
+
+// Pass 1: directions of every particle; departures, arrival counts, touched voxels and the
+// contention test.  Also marks the voxels whose reaction seed itime + x*y + z is 0 this frame.
+template <int KT, int NT>
+__device__ __forceinline__ void ref_sp_directions_body(const RefParams& p, const RefSparse& sp, const uint8_t* slots,
+                                                       const uint32_t* occ, uint32_t itime, uint32_t* diag,
+                                                       uint32_t* contended, const RefRange& R, const float* Pt) {
+    const uint32_t K = KT ? (uint32_t)KT : p.K;
+    const uint32_t XY = p.X * p.Y, step = gridDim.x * NT, dx = step / p.Y, dy = step - dx * p.Y;
+    {
+        uint32_t g = blockIdx.x * NT + threadIdx.x, x = g / p.Y, y = g - x * p.Y;
+        for (; g < XY; g += step) {
+            const uint32_t z = 0u - itime - x * y;  // u32 wrap, as the shader's seed arithmetic
+            if (z < p.Z) set_bit(sp.touch, g * p.Z + z);
+            x += dx;
+            y += dy;
+            if (y >= p.Y) {
+                y -= p.Y;
+                x++;
             }
         }
-        if (!has_dep) continue;
-        rs_store(sp.dirs + (size_t)v * K, K, dr);
-        rs_store(sp.snap + (size_t)v * K, K, sl);
-        set_bit(sp.dep_bm, v);
-        set_bit(sp.touch_bm, v);
-        for (uint32_t s = 0; s < K; s++) {
-            const uint32_t ds = rs_get(dr, s);
-            if (ds >= 6u) continue;
-            const uint32_t w = (uint32_t)((int64_t)v + ref_nb_offset(p, (int)ds));
-            const uint32_t before = atomicAdd(sp.arrivals + w, 1u);
-            const RefSlots ws = rs_load(slots + (size_t)w * K, K);
-            uint32_t nnz = 0;
-            for (uint32_t t = 0; t < K; t++) nnz += rs_get(ws, t) != 0u;
-            const uint32_t ow = occ[w];
-            const uint32_t base = ow > nnz ? ow : nnz;
-            if ((uint64_t)base + before + 1u > K) atomicOr(contended, 1u);
-            set_bit(sp.touch_bm, w);
-        }
     }
-}
-
-__global__ void __launch_bounds__(256) ref_sp_directions(RefParams p, RefSparse sp, const uint8_t* __restrict__ slots,
-                                                         const uint32_t* __restrict__ occ,
-                                                         const uint32_t* __restrict__ itimes, uint32_t step,
-                                                         uint32_t* diag, uint32_t* contended, uint32_t stage_P) {
-    ref_pdl_start();
-    ref_sp_directions_body(p, sp, slots, occ, itimes, step, diag, contended, stage_P);
+    for (uint32_t w0 = blockIdx.x * sp.cw; w0 < sp.W; w0 += gridDim.x * sp.cw) {
+        const uint32_t i = w0 + threadIdx.x;
+        const bool own = threadIdx.x < sp.cw && i < sp.W;
+        const uint32_t m = own ? sp.act[i] : 0u;
+        if (own) {
+            R.area[RW_A][threadIdx.x] = m ? sp.tidy[i] : 0u;
+            R.area[RW_B][threadIdx.x] = m ? __ldg(sp.same + i) : 0u;
+            R.area[RW_C][threadIdx.x] = 0u;  // departures
+        }
+        const uint32_t n = ref_list<NT>(m, R);
+        for (uint32_t e = threadIdx.x; e < n; e += NT) {
+            const uint32_t idx = R.list[e] >> 5, b = R.list[e] & 31u, bit = 1u << b;
+            const uint32_t v = (w0 + idx) * 32u + b;
+            const RefSlots sl = rk_load<KT>(slots, v, K);
+            RefMask full = rs_full(sl);
+            if (!(R.area[RW_A][idx] & bit)) {
+                uint32_t o = occ[v];
+                if (o > K) {
+                    // the gather's contention test fails for this voxel whatever arrives
+                    atomicAdd(diag + DIAG_OCC_RANGE, 1u);
+                    atomicOr(contended, 1u);
+                    o = K;
+                }
+                const RefMask below = rs_valid(o);  // slots past the occupancy don't move
+                full.lo &= below.lo;
+                full.hi &= below.hi;
+            } else if (rm_any(full)) {
+                // a tidy voxel's occupancy is the number of its particles, wherever they lie
+                const RefMask below = rs_valid(rm_count(full));
+                full.lo &= below.lo;
+                full.hi &= below.hi;
+            }
+            if (!rm_any(full)) continue;
+            uint32_t x, y, z;
+            ref_coords(p, v, x, y, z);
+            const uint8_t* reg = p.regions;
+            uint32_t rn[7];
+            rn[0] = reg[v];
+            if (R.area[RW_B][idx] & bit) {
+#pragma unroll
+                for (int k = 1; k < 7; k++) rn[k] = rn[0];
+            } else {
+#pragma unroll
+                for (int k = 1; k < 7; k++) rn[k] = 0u;
+                if (x > 0u) rn[1] = reg[v - p.YZ];
+                if (x < p.X - 1u) rn[2] = reg[v + p.YZ];
+                if (y > 0u) rn[3] = reg[v - p.Z];
+                if (y < p.Y - 1u) rn[4] = reg[v + p.Z];
+                if (z > 0u) rn[5] = reg[v - 1];
+                if (z < p.Z - 1u) rn[6] = reg[v + 1];
+            }
+            RefSlots dr{0x0707070707070707ull, 0x0707070707070707ull};  // 7: stays
+            RefMask leave{0ull, 0ull};
+            for (; rm_any(full); rm_drop(full)) {
+                const uint32_t s = rm_first(full);
+                const int d = ref_decide_rn(p, Pt, rn, x, y, z, rs_get(sl, s), v * K + s, itime);
+                if (d >= 6) continue;
+                rs_set(dr, s, (uint32_t)d);
+                if (s < 8u) leave.lo |= 0x80ull << (8u * s);
+                else leave.hi |= 0x80ull << (8u * (s - 8u));
+            }
+            if (!rm_any(leave)) continue;
+            rk_store<KT>(sp.dirs, v, K, dr);
+            rk_store<KT>(sp.snap, v, K, sl);
+            atomicOr(&R.area[RW_C][idx], bit);
+            for (; rm_any(leave); rm_drop(leave)) {
+                const uint32_t w = (uint32_t)((int64_t)v + ref_nb_offset(p, (int)rs_get(dr, rm_first(leave))));
+                const uint32_t before = atomicAdd(sp.arrivals + w, 1u);
+                set_bit(sp.touch, w);
+                const uint32_t nnz = rs_count(rk_load<KT>(slots, w, K));
+                uint32_t base = nnz;
+                if (!bit_of(sp.tidy, w)) {
+                    const uint32_t ow = occ[w];
+                    base = ow > nnz ? ow : nnz;
+                }
+                if ((uint64_t)base + before + 1u > K) atomicOr(contended, 1u);
+            }
+        }
+        __syncthreads();
+        if (own) {
+            const uint32_t d = R.area[RW_C][threadIdx.x];
+            if (d) {
+                sp.dep[i] = d;
+                atomicOr(sp.touch + i, d);
+            }
+        }
+        __syncthreads();
+    }
 }
 
 // Pass 2 (frames without contention): the gather of every touched voxel, in place.
-__device__ __forceinline__ void ref_sp_gather_body(RefParams p, RefSparse sp, uint8_t* slots, uint32_t* occ,
-                                                   int32_t* conc, const uint32_t* contended) {
-    if (*contended) return;
-    const uint32_t K = p.K, S1 = p.S1;
-    const uint32_t n = __ldcg(sp.cnt + 1);
-    for (uint32_t e = grid_tid(); e < n; e += grid_threads()) {
-        const uint32_t w = sp.touch_list[e];
-        sp.arrivals[w] = 0u;
-        uint32_t x, y, z;
-        ref_coords(p, w, x, y, z);
-        const bool has_nb[6] = {x > 0u, x < p.X - 1u, y > 0u, y < p.Y - 1u, z > 0u, z < p.Z - 1u};
-        RefSlots sl = rs_load(slots + (size_t)w * K, K);
-        uint32_t o = occ[w];
-        int32_t* cw = conc + (size_t)w * S1;
-        // arrivals from the neighbour on `side`: the particles it moves in direction side ^ 1
-        auto arrive = [&](int side) {
-            if (!has_nb[side]) return;
-            const uint32_t u = (uint32_t)((int64_t)w + ref_nb_offset(p, side));
-            if (!bit_of(sp.dep_bm, u)) return;
-            const uint32_t want = (uint32_t)(side ^ 1);
-            const RefSlots nd = rs_load(sp.dirs + (size_t)u * K, K);
-            const RefSlots ns = rs_load(sp.snap + (size_t)u * K, K);
-            for (uint32_t s = 0; s < K; s++) {
-                if (rs_get(nd, s) != want) continue;
-                const uint32_t q = rs_get(ns, s);
-                uint32_t j = 0;
-                while (j < K && rs_get(sl, j) != 0u) j++;
-                if (j == K) continue;  // unreachable without contention
-                rs_set(sl, j, q);
-                o++;
-                cw[q] = (int32_t)((uint32_t)cw[q] + 1u);
-            }
-        };
-        arrive(0);  // from -x
-        arrive(2);  // from -y
-        arrive(4);  // from -z
-        if (bit_of(sp.dep_bm, w)) {
-            const RefSlots nd = rs_load(sp.dirs + (size_t)w * K, K);
-            for (uint32_t s = 0; s < K; s++) {
-                if (rs_get(nd, s) >= 6u) continue;
-                const uint32_t q = rs_get(sl, s);
-                rs_set(sl, s, 0u);
-                o--;
-                cw[q] = (int32_t)((uint32_t)cw[q] - 1u);
-            }
+template <int KT, int NT>
+__device__ __forceinline__ void ref_sp_gather_body(const RefParams& p, const RefSparse& sp, uint8_t* slots, uint32_t* occ,
+                                                   int32_t* conc, const RefRange& R) {
+    const uint32_t K = KT ? (uint32_t)KT : p.K, S1 = p.S1;
+    const RefMask valid = rs_valid(K);
+    for (uint32_t w0 = blockIdx.x * sp.cw; w0 < sp.W; w0 += gridDim.x * sp.cw) {
+        const uint32_t i = w0 + threadIdx.x;
+        const bool own = threadIdx.x < sp.cw && i < sp.W;
+        const uint32_t m = own ? ref_word(sp.touch + i) : 0u;
+        if (own) {
+            R.area[RW_A][threadIdx.x] = m ? sp.tidy[i] : 0u;
+            R.area[RW_B][threadIdx.x] = m ? ref_word(sp.dep + i) : 0u;
         }
-        arrive(5);  // from +z
-        arrive(3);  // from +y
-        arrive(1);  // from +x
-        rs_store(slots + (size_t)w * K, K, sl);
-        occ[w] = o;
+        const uint32_t n = ref_list<NT>(m, R);
+        for (uint32_t e = threadIdx.x; e < n; e += NT) {
+            const uint32_t idx = R.list[e] >> 5, b = R.list[e] & 31u, bit = 1u << b;
+            const uint32_t w = (w0 + idx) * 32u + b;
+            uint32_t x, y, z;
+            ref_coords(p, w, x, y, z);
+            const bool has_nb[6] = {x > 0u, x < p.X - 1u, y > 0u, y < p.Y - 1u, z > 0u, z < p.Z - 1u};
+            // the departure words of all six sides, then the snapshots of those that left, each in flight together
+            bool from[6];
+#pragma unroll
+            for (int s = 0; s < 6; s++) {
+                const uint32_t u = has_nb[s] ? (uint32_t)((int64_t)w + ref_nb_offset(p, s)) : w;
+                from[s] = has_nb[s] && bit_of(sp.dep, u);
+            }
+            RefSlots sl = rk_load<KT>(slots, w, K);
+            RefSlots nd[6], ns[6];
+            const bool leaves = R.area[RW_B][idx] & bit;
+            RefSlots own_d{0x0707070707070707ull, 0x0707070707070707ull};
+            if (leaves) own_d = rk_load<KT>(sp.dirs, w, K);
+#pragma unroll
+            for (int s = 0; s < 6; s++) {
+                nd[s] = ns[s] = RefSlots{0ull, 0ull};
+                if (!from[s]) continue;
+                const uint32_t u = (uint32_t)((int64_t)w + ref_nb_offset(p, s));
+                nd[s] = rk_load<KT>(sp.dirs, u, K);
+                ns[s] = rk_load<KT>(sp.snap, u, K);
+            }
+            sp.arrivals[w] = 0u;
+            const bool tidy = R.area[RW_A][idx] & bit;
+            int32_t* const cw = conc + (size_t)w * S1;
+            uint32_t o = tidy ? 0u : occ[w];
+            // arrivals from the neighbour on side `s`: the particles it moves in direction s ^ 1
+            auto arrive = [&](int s) {
+                if (!from[s]) return;
+                const uint64_t want = (uint64_t)(uint32_t)(s ^ 1) * 0x0101010101010101ull;
+                RefMask mv{~bytes_nonzero(nd[s].lo ^ want) & valid.lo, ~bytes_nonzero(nd[s].hi ^ want) & valid.hi};
+                for (; rm_any(mv); rm_drop(mv)) {
+                    const uint32_t q = rs_get(ns[s], rm_first(mv));
+                    const RefMask full = rs_full(sl);
+                    const RefMask room{~full.lo & valid.lo, ~full.hi & valid.hi};
+                    if (!rm_any(room)) continue;  // unreachable without contention
+                    rs_set(sl, rm_first(room), q);
+                    if (!tidy) {
+                        o++;
+                        cw[q] = (int32_t)((uint32_t)cw[q] + 1u);
+                    }
+                }
+            };
+            arrive(0);  // from -x
+            arrive(2);  // from -y
+            arrive(4);  // from -z
+            if (leaves) {
+                // direction bytes below 6 (they are at most 7)
+                RefMask mv{~(own_d.lo + 0x7A7A7A7A7A7A7A7Aull) & valid.lo, ~(own_d.hi + 0x7A7A7A7A7A7A7A7Aull) & valid.hi};
+                for (; rm_any(mv); rm_drop(mv)) {
+                    const uint32_t s = rm_first(mv), q = rs_get(sl, s);
+                    rs_set(sl, s, 0u);
+                    if (!tidy) {
+                        o--;
+                        cw[q] = (int32_t)((uint32_t)cw[q] - 1u);
+                    }
+                }
+            }
+            arrive(5);  // from +z
+            arrive(3);  // from +y
+            arrive(1);  // from +x
+            rk_store<KT>(slots, w, K, sl);
+            if (!tidy) occ[w] = o;
+        }
+        __syncthreads();
     }
 }
 
-__global__ void __launch_bounds__(256) ref_sp_gather(RefParams p, RefSparse sp, uint8_t* __restrict__ slots,
-                                                     uint32_t* __restrict__ occ, int32_t* __restrict__ conc,
-                                                     const uint32_t* __restrict__ contended) {
-    ref_pdl_start();
-    ref_sp_gather_body(p, sp, slots, occ, conc, contended);
-}
-
-// Pass 3 (contended frames): the serial diffusion of rdme.wgsl:45-88 in place,
-// voxels in linear order.  A departing slot still holds its particle when its
-// voxel's turn comes (arrivals only fill empty slots), and a slot that an
-// arrival filled has direction 7.  One block scans the departure bitmap; its
-// first thread makes the moves.
-__device__ __forceinline__ void ref_sp_serial_body(RefParams p, RefSparse sp, uint8_t* slots, uint32_t* occ,
-                                                   int32_t* conc, uint32_t* diag, const uint32_t* contended) {
-    if (*contended == 0u) return;
-    __shared__ uint32_t s_words[1024];
+// Pass 2 of contended frames: the serial diffusion of rdme.wgsl:45-88 in place, voxels in linear
+// order.  A departing slot still holds its particle when its voxel's turn comes (arrivals only fill
+// empty slots), and a slot that an arrival filled has direction 7.  One block scans the departure
+// bitmap; its first thread makes the moves.  A move changes slots, occupancy and counts alike, so a
+// tidy voxel stays tidy.
+__device__ __forceinline__ void ref_sp_serial_body(const RefParams& p, const RefSparse& sp, uint8_t* slots, uint32_t* occ,
+                                                   int32_t* conc, uint32_t* diag, uint32_t* s_words) {
     const uint32_t K = p.K, S1 = p.S1;
     uint32_t spills = 0;
     for (uint32_t w0 = 0; w0 < sp.W; w0 += blockDim.x) {
         const uint32_t i = w0 + threadIdx.x;
-        s_words[threadIdx.x] = i < sp.W ? sp.dep_bm[i] : 0u;
+        s_words[threadIdx.x] = i < sp.W ? ref_word(sp.dep + i) : 0u;
         __syncthreads();
         if (threadIdx.x == 0) {
             for (uint32_t k = 0; k < blockDim.x && w0 + k < sp.W; k++) {
@@ -741,17 +838,22 @@ __device__ __forceinline__ void ref_sp_serial_body(RefParams p, RefSparse sp, ui
                         if (d >= 6) continue;
                         const uint32_t w = (uint32_t)((int64_t)v + ref_nb_offset(p, d));
                         sp.arrivals[w] = 0u;
-                        if (occ[w] >= K) { spills++; continue; }
+                        const bool tw = bit_of(sp.tidy, w);
+                        if (!tw && occ[w] >= K) { spills++; continue; }
                         uint32_t j = 0;
                         while (j < K && slots[(size_t)w * K + j] != 0) j++;
                         if (j == K) { spills++; continue; }
                         const uint8_t q = slots[(size_t)v * K + s];
                         slots[(size_t)w * K + j] = q;
-                        occ[w] += 1u;
-                        conc[(size_t)w * S1 + q] = (int32_t)((uint32_t)conc[(size_t)w * S1 + q] + 1u);
-                        occ[v] -= 1u;
+                        if (!tw) {
+                            occ[w] += 1u;
+                            conc[(size_t)w * S1 + q] = (int32_t)((uint32_t)conc[(size_t)w * S1 + q] + 1u);
+                        }
                         slots[(size_t)v * K + s] = 0;
-                        conc[(size_t)v * S1 + q] = (int32_t)((uint32_t)conc[(size_t)v * S1 + q] - 1u);
+                        if (!bit_of(sp.tidy, v)) {
+                            occ[v] -= 1u;
+                            conc[(size_t)v * S1 + q] = (int32_t)((uint32_t)conc[(size_t)v * S1 + q] - 1u);
+                        }
                     }
                 }
             }
@@ -764,54 +866,99 @@ __device__ __forceinline__ void ref_sp_serial_body(RefParams p, RefSparse sp, ui
     }
 }
 
-__global__ void ref_sp_serial(RefParams p, RefSparse sp, uint8_t* __restrict__ slots, uint32_t* __restrict__ occ,
-                              int32_t* __restrict__ conc, uint32_t* diag, const uint32_t* __restrict__ contended) {
-    ref_pdl_start();
-    ref_sp_serial_body(p, sp, slots, occ, conc, diag, contended);
-}
-
-// The reaction pass on one voxel and its bit in act bitmap c ^ 1.
-// The reaction tables of ref_cme_voxel staged in shared memory by the reaction pass.
+// The reaction tables staged in shared memory by the reaction pass.
 struct RefTables {
     const uint32_t* reactants;  // [R+1][3]
     const float* rates;         // [R+1]
     const int32_t* stoich;      // [R+1][S1]
+    const uint32_t* uses;       // [S1][UW]
+    const float* fire1;         // [S1]
 };
+__host__ __device__ constexpr size_t ref_table_words(uint32_t S1, uint32_t R, uint32_t UW) {
+    return 4 * ((size_t)R + 1) + ((size_t)R + 1) * S1 + (size_t)S1 * UW + S1;
+}
+__device__ __forceinline__ RefTables ref_stage_tables(const RefParams& p, const RefSparse& sp, uint32_t* sm) {
+    uint32_t* const s_re = sm;
+    float* const s_rate = reinterpret_cast<float*>(s_re + 3 * (p.R + 1));
+    int32_t* const s_st = reinterpret_cast<int32_t*>(s_rate + (p.R + 1));
+    uint32_t* const s_uses = reinterpret_cast<uint32_t*>(s_st + (p.R + 1) * p.S1);
+    float* const s_fire = reinterpret_cast<float*>(s_uses + p.S1 * sp.UW);
+    for (uint32_t i = threadIdx.x; i < 3 * (p.R + 1); i += blockDim.x) s_re[i] = p.reactants[i];
+    for (uint32_t i = threadIdx.x; i < p.R + 1; i += blockDim.x) s_rate[i] = p.rates[i];
+    for (uint32_t i = threadIdx.x; i < (p.R + 1) * p.S1; i += blockDim.x) s_st[i] = p.stoich[i];
+    for (uint32_t i = threadIdx.x; i < p.S1 * sp.UW; i += blockDim.x) s_uses[i] = sp.uses[i];
+    for (uint32_t i = threadIdx.x; i < p.S1; i += blockDim.x) s_fire[i] = sp.fire1[i];
+    return RefTables{s_re, s_rate, s_st, s_uses, s_fire};
+}
 
-// ref_cme_voxel with the tables in shared memory (T) and the voxel's concentration row copied into
-// the thread's shared-memory row `row` while it is evaluated (every change is written through to
-// the global row): the same operations in the same order, so the same results, with the
-// propensity and selection loops reading shared memory instead of about a hundred dependent
-// global loads per voxel.
-__device__ __forceinline__ void ref_cme_voxel_rows(const RefParams& p, const RefTables& T, uint64_t v,
-                                                   uint8_t* __restrict__ slots, uint32_t* __restrict__ occ,
-                                                   int32_t* __restrict__ conc, uint32_t itime, int32_t* s_delta,
-                                                   int32_t* row) {
-    const uint32_t K = p.K, S1 = p.S1, R = p.R;
-    const uint32_t S = S1 - 1;
+// The reaction pass on voxel v (tidy or not), as ref_cme_voxel; `row` is the thread's shared-memory
+// concentration row.  Returns whether the voxel stays in act; `tidy` as it is afterwards.
+template <int KT>
+__device__ __forceinline__ bool ref_react(const RefParams& p, const RefSparse& sp, const RefTables& T, uint32_t v,
+                                          uint8_t* slots, uint32_t* occ, int32_t* conc, uint32_t itime,
+                                          int32_t* s_delta, int32_t* row, bool& tidy) {
+    const uint32_t K = KT ? (uint32_t)KT : p.K, S1 = p.S1, R = p.R, S = S1 - 1u;
+    const RefSlots snap = rk_load<KT>(slots, v, K);
     uint32_t x, y, z;
-    ref_coords(p, (uint32_t)v, x, y, z);
-    int32_t* c = conc + v * S1;
-    for (uint32_t s = 0; s < S1; s++) row[s] = c[s];
-    if (row[0] != 1) {  // stored only when it changes: an unchanged row is not written back
-        row[0] = 1;
-        c[0] = 1;
-    }
+    ref_coords(p, v, x, y, z);
+    const uint32_t state = d_pcg(itime + x * y + z);
+    const float r1 = d_uniform_float(state);
+    RefMask full = rs_full(snap);
+    const uint32_t n = rm_count(full);
+    const bool was = tidy;
+    RefSlots sl = snap;
+    bool fires;
+    bool have_row = false;
+    int32_t* const c = conc + (size_t)v * S1;
+    auto make_row = [&]() {
+        have_row = true;
+        if (was) {
+            row[0] = 1;
+            for (uint32_t s = 1; s < S1; s++) row[s] = 0;
+            for (RefMask f = full; rm_any(f); rm_drop(f)) row[rs_get(snap, rm_first(f))]++;
+        } else {
+            for (uint32_t s = 0; s < S1; s++) row[s] = c[s];
+            if (row[0] != 1) {
+                row[0] = 1;
+                c[0] = 1;
+            }
+        }
+    };
     auto prop_of = [&](uint32_t r) -> float {
         const uint32_t prod = (uint32_t)row[T.reactants[r * 3]] * (uint32_t)row[T.reactants[r * 3 + 1]] *
                               (uint32_t)row[T.reactants[r * 3 + 2]];
         return __fmul_rn(T.rates[r], __int2float_rn((int32_t)prod));
     };
     float total = 0.0f;
-    for (uint32_t r = 1; r <= R; r++) total = __fadd_rn(total, prop_of(r));
-    const RefSlots snap = rs_load(slots + v * K, K);
-    RefSlots sl = snap;
-    uint32_t state = d_pcg(itime + x * y + z);
-    float r1 = d_uniform_float(state);
-    float fire_p = __fsub_rn(1.0f, d_expf(__fmul_rn(-total, p.tau)));
-    if (r1 <= fire_p) {
+    auto sum = [&]() {
+        total = 0.0f;
+        if (sp.finite) {  // a reaction that lacks a reactant adds a zero, which changes no sum
+            for (uint32_t u = 0; u < sp.UW; u++) {
+                uint32_t m = 0xFFFFFFFFu;
+                for (uint32_t s = 1; s < S1; s++)
+                    if (row[s] == 0) m &= ~T.uses[s * sp.UW + u];
+                if (u == 0u) m &= ~1u;
+                if (32u * u + 31u > R) m &= R >= 32u * u ? (2u << (R - 32u * u)) - 1u : 0u;
+                for (; m; m &= m - 1u) total = __fadd_rn(total, prop_of(32u * u + (uint32_t)(__ffs((int)m) - 1)));
+            }
+        } else {
+            for (uint32_t r = 1; r <= R; r++) total = __fadd_rn(total, prop_of(r));
+        }
+    };
+    if (was && n <= 1u) {
+        fires = r1 <= T.fire1[n ? rs_get(snap, rm_first(full)) : 0u];
+    } else {
+        make_row();
+        sum();
+        fires = r1 <= __fsub_rn(1.0f, d_expf(__fmul_rn(-total, p.tau)));
+    }
+    if (fires) {
+        if (!have_row) {
+            make_row();
+            sum();
+        }
         atomicAdd(&s_delta[S1], 1);
-        float r2 = d_uniform_float(state + 1u);
+        const float r2 = d_uniform_float(state + 1u);
         // selection over cum[i] = cum[i-1] + a_i, normalised for i < R (cme.wgsl:50-52,70-73)
         uint32_t i = 0;
         float run = 0.0f;
@@ -822,15 +969,15 @@ __device__ __forceinline__ void ref_cme_voxel_rows(const RefParams& p, const Ref
         }
         const int32_t* st = T.stoich + (size_t)i * S1;
         uint32_t j = 0;
-        int32_t new_occ = (int32_t)occ[v];
-        uint64_t ri = v * K;  // reservoirs[idx_lattice], cme.wgsl:80
-        uint32_t resv = (ri < p.V) ? p.reservoir[ri] : 0u;
+        const int32_t occ0 = was ? (int32_t)n : (int32_t)occ[v];
+        int32_t new_occ = occ0;
+        const uint64_t ri = (uint64_t)v * K;  // reservoirs[idx_lattice], cme.wgsl:80
+        const uint32_t resv = (ri < p.V) ? p.reservoir[ri] : 0u;
         bool rolled = false;
         for (uint32_t s = 1; s <= S && !rolled; s++) {
             if (resv == s) continue;
-            int32_t d = st[s];
+            const int32_t d = st[s];
             row[s] = (int32_t)((uint32_t)row[s] + (uint32_t)d);
-            if (d) c[s] = row[s];
             new_occ = (int32_t)((uint32_t)new_occ + (uint32_t)d);
             if (d) atomicAdd(&s_delta[s], d);
             int32_t cc = row[s];
@@ -841,12 +988,9 @@ __device__ __forceinline__ void ref_cme_voxel_rows(const RefParams& p, const Ref
                 if (j >= K) {
                     sl = snap;
                     for (uint32_t s2 = 1; s2 <= s; s2++) {
-                        int32_t d2 = st[s2];
+                        const int32_t d2 = st[s2];
                         row[s2] = (int32_t)((uint32_t)row[s2] - (uint32_t)d2);
-                        if (d2) {
-                            c[s2] = row[s2];
-                            atomicAdd(&s_delta[s2], -d2);
-                        }
+                        if (d2) atomicAdd(&s_delta[s2], -d2);
                     }
                     atomicAdd(&s_delta[S1 + 1], 1);
                     rolled = true;
@@ -855,153 +999,403 @@ __device__ __forceinline__ void ref_cme_voxel_rows(const RefParams& p, const Ref
             }
         }
         if (!rolled) {
-            occ[v] = (uint32_t)new_occ;
             while (j < K) rs_set(sl, j++, 0u);
+        } else {
+            new_occ = occ0;
         }
+        // do the new slots still imply the occupancy and the counts?
+        const RefMask f1 = rs_full(sl);
+        bool same = new_occ == (int32_t)rm_count(f1);
+        for (RefMask f = f1; rm_any(f); rm_drop(f)) row[rs_get(sl, rm_first(f))]--;
+        for (uint32_t s = 1; s < S1; s++) same &= row[s] == 0;
+        for (RefMask f = f1; rm_any(f); rm_drop(f)) row[rs_get(sl, rm_first(f))]++;
+        tidy = same;
+        if (!same) {
+            for (uint32_t s = 0; s < S1; s++) c[s] = row[s];
+            occ[v] = (uint32_t)new_occ;
+        }
+        full = f1;
     }
     // stable move of the non-zero slots to the front
-    RefSlots out{0ull, 0ull};
-    uint32_t jj = 0;
-    for (uint32_t s = 0; s < K; s++) {
-        const uint32_t q = rs_get(sl, s);
-        if (q != 0u) rs_set(out, jj++, q);
+    auto packed = [](uint64_t f) -> bool {  // bytes marked from the lowest on
+        const uint64_t t = f | (f - (f >> 7));
+        return (t & (t + 1ull)) == 0ull;
+    };
+    RefSlots out = sl;
+    if (!(packed(full.lo) && packed(full.hi) && (full.hi == 0ull || full.lo == 0x8080808080808080ull))) {
+        out = RefSlots{0ull, 0ull};
+        uint32_t jj = 0;
+        for (RefMask f = full; rm_any(f); rm_drop(f)) rs_set(out, jj++, rs_get(sl, rm_first(f)));
     }
-    if (out.lo != snap.lo || out.hi != snap.hi) rs_store(slots + v * K, K, out);
+    if (out.lo != snap.lo || out.hi != snap.hi) rk_store<KT>(slots, v, K, out);
+    bool keep = rm_any(full);
+    if (!tidy && !keep) {
+        keep = occ[v] != 0u;
+        for (uint32_t s = 1; s < S1 && !keep; s++) keep |= row[s] != 0;
+    }
+    return keep;
 }
 
-// rows: the staged tables T and the thread's shared-memory concentration row `row` are used (else,
-// when they do not fit, the global-memory form)
-__device__ __forceinline__ void ref_sp_react(const RefParams& p, const RefSparse& sp, uint32_t v, uint8_t* slots,
-                                             uint32_t* occ, int32_t* conc, uint32_t itime, int32_t* s_delta,
-                                             bool rows, const RefTables& T, int32_t* row) {
-    const uint32_t K = p.K, S1 = p.S1;
-    const int32_t* c = conc + (size_t)v * S1;
-    if (rows) {
-        ref_cme_voxel_rows(p, T, v, slots, occ, conc, itime, s_delta, row);
-        c = row;
-    } else {
-        ref_cme_voxel(p, v, slots, occ, conc, itime, s_delta);
+// Pass 3: the reaction pass over act and touch (every voxel when `dense`), which leaves the next
+// frame's act words and clears the touch and departure words.  rows: the staged tables and a
+// shared-memory row per thread are used (else, when they do not fit, the global-memory form; no
+// voxel is tidy then).
+template <int KT, int NT>
+__device__ __forceinline__ void ref_sp_cme_body(const RefParams& p, const RefSparse& sp, uint8_t* slots, uint32_t* occ,
+                                                int32_t* conc, uint32_t itime, uint32_t dense, const RefRange& R,
+                                                const RefTables& T, int32_t* s_delta, int32_t* row, uint32_t rows) {
+    const uint32_t K = KT ? (uint32_t)KT : p.K;
+    for (uint32_t w0 = blockIdx.x * sp.cw; w0 < sp.W; w0 += gridDim.x * sp.cw) {
+        const uint32_t i = w0 + threadIdx.x;
+        const bool own = threadIdx.x < sp.cw && i < sp.W;
+        uint32_t m = 0u, a = 0u, t = 0u, tidy0 = 0u;
+        if (own) {
+            a = sp.act[i];
+            t = ref_word(sp.touch + i);
+            tidy0 = sp.tidy[i];
+            m = a | t;
+            if (dense) m = (uint64_t)i * 32u + 32u <= p.V ? 0xFFFFFFFFu : (1u << (p.V & 31u)) - 1u;
+            R.area[RW_A][threadIdx.x] = tidy0;
+            R.area[RW_B][threadIdx.x] = 0u;   // the next act word
+            R.area[RW_C][threadIdx.x] = tidy0;  // the next tidy word
+        }
+        const uint32_t n = ref_list<NT>(m, R);
+        for (uint32_t e = threadIdx.x; e < n; e += NT) {
+            const uint32_t idx = R.list[e] >> 5, b = R.list[e] & 31u, bit = 1u << b;
+            const uint32_t v = (w0 + idx) * 32u + b;
+            bool keep;
+            if (rows) {
+                const bool was = R.area[RW_A][idx] & bit;
+                bool tidy = was;
+                keep = ref_react<KT>(p, sp, T, v, slots, occ, conc, itime, s_delta, row, tidy);
+                if (tidy != was) atomicXor(&R.area[RW_C][idx], bit);
+            } else {
+                ref_cme_voxel(p, v, slots, occ, conc, itime, s_delta);
+                keep = occ[v] != 0u || rm_any(rs_full(rk_load<KT>(slots, v, K)));
+                for (uint32_t s = 1; s < p.S1 && !keep; s++) keep |= conc[(size_t)v * p.S1 + s] != 0;
+            }
+            if (keep) atomicOr(&R.area[RW_B][idx], bit);
+        }
+        __syncthreads();
+        if (own) {
+            const uint32_t keep = R.area[RW_B][threadIdx.x], tidy = R.area[RW_C][threadIdx.x];
+            if (keep != a) sp.act[i] = keep;
+            if (tidy != tidy0) sp.tidy[i] = tidy;
+            if (t) {
+                sp.touch[i] = 0u;
+                sp.dep[i] = 0u;  // a voxel with a departure is touched
+            }
+        }
+        __syncthreads();
     }
-    const RefSlots sl = rs_load(slots + (size_t)v * K, K);
-    bool keep = occ[v] != 0u || (sl.lo | sl.hi) != 0ull;
-    for (uint32_t s = 1; s < S1 && !keep; s++) keep |= c[s] != 0;
-    if (keep) set_bit(act_next(sp), v);
 }
 
-// Pass 4: the reaction pass over the union list (every voxel when `dense`),
-// setting act bitmap c ^ 1; clears the contention flag, the touch and
-// departure bitmaps and the act list counter for the next frame.
-__device__ __forceinline__ void ref_sp_cme_body(RefParams p, RefSparse sp, uint8_t* slots, uint32_t* occ,
-                                                int32_t* conc, const uint32_t* itimes, uint32_t step, uint32_t dense,
-                                                int32_t* stat, uint32_t* diag, uint32_t* contended, uint32_t rows) {
-    extern __shared__ int32_t s_delta[];  // [S1] + 2 counters, then (rows) the tables and the rows
-    for (uint32_t s = threadIdx.x; s < p.S1 + 2; s += blockDim.x) s_delta[s] = 0;
-    if (grid_tid() == 0) {
-        *contended = 0u;  // every reader of this frame's flag has run
-        sp.cnt[0] = 0u;
-    }
-    RefTables T{};
-    int32_t* row = nullptr;
-    if (rows) {
-        uint32_t* s_re = reinterpret_cast<uint32_t*>(s_delta + p.S1 + 2);
-        float* s_rate = reinterpret_cast<float*>(s_re + 3 * (p.R + 1));
-        int32_t* s_st = reinterpret_cast<int32_t*>(s_rate + (p.R + 1));
-        for (uint32_t i = threadIdx.x; i < 3 * (p.R + 1); i += blockDim.x) s_re[i] = p.reactants[i];
-        for (uint32_t i = threadIdx.x; i < p.R + 1; i += blockDim.x) s_rate[i] = p.rates[i];
-        for (uint32_t i = threadIdx.x; i < (p.R + 1) * p.S1; i += blockDim.x) s_st[i] = p.stoich[i];
-        T = RefTables{s_re, s_rate, s_st};
-        row = s_st + (p.R + 1) * p.S1 + threadIdx.x * p.S1;
-    }
-    __syncthreads();
+// Threads of a block of the three launches.
+constexpr int REF_NT = 128;
+constexpr size_t REF_SMEM = 44u * 1024u;  // dynamic shared memory of a launch without an attribute, and some for static
+
+template <int KT>
+__global__ void __launch_bounds__(REF_NT) ref_sp_directions(const __grid_constant__ RefParams p,
+                                                            const __grid_constant__ RefSparse sp, const uint8_t* slots,
+                                                            const uint32_t* occ, const uint32_t* itimes, uint32_t step,
+                                                            uint32_t* diag, uint32_t* contended, uint32_t stage_P) {
+    extern __shared__ __align__(16) uint32_t sm[];
+    float* const s_P = reinterpret_cast<float*>(sm + ref_range_words(sp.cw));
+    ref_allow_next();
+    ref_stage_P(p, s_P, stage_P);
     const uint32_t itime = __ldg(itimes + step);
-    for (uint32_t i = grid_tid(); i < sp.W; i += grid_threads()) {
-        sp.touch_bm[i] = 0u;
-        sp.dep_bm[i] = 0u;
-    }
-    if (dense) {
-        for (uint32_t v = grid_tid(); v < (uint32_t)p.V; v += grid_threads())
-            ref_sp_react(p, sp, v, slots, occ, conc, itime, s_delta, rows != 0u, T, row);
-    } else {
-        const uint32_t n = __ldcg(sp.cnt + 2);
-        for (uint32_t e = grid_tid(); e < n; e += grid_threads())
-            ref_sp_react(p, sp, sp.union_list[e], slots, occ, conc, itime, s_delta, rows != 0u, T, row);
-    }
-    __syncthreads();
-    ref_flush_block(p, s_delta, stat, diag);
+    ref_wait_previous();
+    ref_sp_directions_body<KT, REF_NT>(p, sp, slots, occ, itime, diag, contended, ref_range(sm, sp.cw), stage_P ? s_P : p.P);
 }
 
-__global__ void __launch_bounds__(256) ref_sp_cme(RefParams p, RefSparse sp, uint8_t* __restrict__ slots,
-                                                  uint32_t* __restrict__ occ, int32_t* __restrict__ conc,
-                                                  const uint32_t* __restrict__ itimes, uint32_t step, uint32_t dense,
-                                                  int32_t* stat, uint32_t* diag, uint32_t* contended, uint32_t rows) {
-    ref_pdl_start();
-    ref_sp_cme_body(p, sp, slots, occ, conc, itimes, step, dense, stat, diag, contended, rows);
+template <int KT>
+__global__ void __launch_bounds__(REF_NT) ref_sp_move(const __grid_constant__ RefParams p,
+                                                      const __grid_constant__ RefSparse sp, uint8_t* slots, uint32_t* occ,
+                                                      int32_t* conc, uint32_t* diag, const uint32_t* contended) {
+    extern __shared__ __align__(16) uint32_t sm[];
+    ref_allow_next();
+    ref_wait_previous();
+    if (ref_word(contended)) {
+        if (blockIdx.x == 0) {
+            __shared__ uint32_t s_words[REF_NT];
+            ref_sp_serial_body(p, sp, slots, occ, conc, diag, s_words);
+        }
+        return;
+    }
+    ref_sp_gather_body<KT, REF_NT>(p, sp, slots, occ, conc, ref_range(sm, sp.cw));
+}
+
+// Shared memory of the reaction pass behind the range: S1 + 2 counters, then (rows) the tables and rows.
+template <int KT>
+__global__ void __launch_bounds__(REF_NT) ref_sp_cme(const __grid_constant__ RefParams p,
+                                                     const __grid_constant__ RefSparse sp, uint8_t* slots, uint32_t* occ,
+                                                     int32_t* conc, const uint32_t* itimes, uint32_t step, uint32_t dense,
+                                                     int32_t* stat, uint32_t* diag, uint32_t* contended, uint32_t rows) {
+    extern __shared__ __align__(16) uint32_t sm[];
+    int32_t* const s_delta = reinterpret_cast<int32_t*>(sm + ref_range_words(sp.cw));
+    ref_allow_next();
+    for (uint32_t s = threadIdx.x; s < p.S1 + 2; s += REF_NT) s_delta[s] = 0;
+    uint32_t* const s_tab = reinterpret_cast<uint32_t*>(s_delta + p.S1 + 2);
+    RefTables T{};
+    if (rows) T = ref_stage_tables(p, sp, s_tab);
+    int32_t* const row = reinterpret_cast<int32_t*>(s_tab + ref_table_words(p.S1, p.R, sp.UW)) + threadIdx.x * p.S1;
+    const uint32_t itime = __ldg(itimes + step);
+    ref_wait_previous();
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *contended = 0u;  // every reader of this frame's flag has run
+    ref_sp_cme_body<KT, REF_NT>(p, sp, slots, occ, conc, itime, dense, ref_range(sm, sp.cw), T, s_delta, row, rows);
+    ref_flush_block(p, s_delta, stat, diag);
 }
 
 // Threads of the one-block form below.
 constexpr int REF_BLOCK_THREADS = 512;
-// Lattices of at most this many voxels run every frame of a call in the one-block form: one SM does
-// such a frame's work sooner than six launches take to run back to back.  Measured on cubic
-// lattices with one particle per 16 voxels: six launches take 31-36 us a frame at any size from
-// 4,096 to 110,592 voxels, the one block 22.9 us at 4,096 and 69.8 us at 13,824 voxels (its time
-// follows the particles).
-constexpr uint64_t REF_BLOCK_MAX_VOXELS = 6144;
+// Lattices of at most this many voxels and (when they are uploaded) particles run every frame of a call
+// in the one-block form, if its state and a row per thread fit in shared memory.  us per frame, one block
+// / three launches: 64 x 64 x 1, K = 8, with 200 particles 9.0 / 12.9, 400 10.0 / 13.5, 800 15.2 / 14.5; 77 x
+// 78 x 1 with 600 13.3 / 13.9, 1,100 19.0 / 14.6; without the rows, 16^3, K = 16, 300 particles 27 / 13.4.  The
+// block's time is one SM's dependent steps (about a dozen barriers and the entries' instruction chains) and
+// follows the particles; the launches' is three launch latencies whatever the size up to about 40^3.  With
+// the state in global memory the block took 12.4 at 400 particles: a frame was a chain of L2 round trips.
+constexpr uint64_t REF_BLOCK_MAX_VOXELS = 6144, REF_BLOCK_MAX_PARTICLES = 600;
 
 // Every frame of a step call in one block: the passes' own bodies in the same order, with block
-// barriers where the launches were (the serial pass runs on the same block).  The bodies read
-// nothing that the block writes through the non-coherent path (their pointers carry no
-// __restrict__ here), so each pass sees the previous one's writes after the barrier.
+// barriers where the launches were (the serial pass runs on the same block).  What the frames read and
+// write (slots, bitmaps, arrivals, directions and snapshots) is in shared memory for the whole call;
+// the occupancy and rows of voxels that are not tidy stay in global memory, and the bodies read
+// nothing that the block writes through the non-coherent path.
+template <int KT>
 __global__ void __launch_bounds__(REF_BLOCK_THREADS, 1)
-    ref_sp_frames_block(RefParams p, RefSparse sp, uint8_t* slots, uint32_t* occ, int32_t* conc,
-                        const uint32_t* itimes, uint32_t step0, uint32_t n, uint32_t dense_first,
-                        uint32_t dense_always, int32_t* stat, uint32_t* diag, uint32_t* contended, uint32_t stage_P,
-                        uint32_t rows) {
+    ref_sp_frames_block(const __grid_constant__ RefParams p, const __grid_constant__ RefSparse g, uint8_t* g_slots,
+                        uint32_t* occ, int32_t* conc, const uint32_t* itimes, uint32_t step0, uint32_t n,
+                        uint32_t dense_first, uint32_t dense_always, int32_t* stat, uint32_t* diag,
+                        uint32_t* g_contended, uint32_t stage_P, uint32_t rows, uint32_t other) {
+    constexpr int NT = REF_BLOCK_THREADS;
+    extern __shared__ __align__(16) uint32_t sm[];
+    __shared__ uint32_t s_words[NT];
+    __shared__ uint32_t s_contended;
+    uint32_t* const contended = &s_contended;
+    // the state, behind `other` bytes of lists and tables
+    RefSparse sp = g;
+    const uint32_t V = (uint32_t)p.V, VK = (uint32_t)(p.V * p.K), VKa = (VK + 15u) & ~15u;
+    uint8_t* const s_state = reinterpret_cast<uint8_t*>(sm) + other;
+    uint8_t* const slots = s_state;
+    sp.dirs = slots + VKa;
+    sp.snap = sp.dirs + VKa;
+    sp.arrivals = reinterpret_cast<uint32_t*>(sp.snap + VKa);
+    sp.act = sp.arrivals + V;
+    sp.touch = sp.act + g.W;
+    sp.dep = sp.touch + g.W;
+    sp.tidy = sp.dep + g.W;
+    for (uint32_t i = threadIdx.x; i < VKa / 4u; i += NT)
+        if (4u * i + 4u <= VK) reinterpret_cast<uint32_t*>(slots)[i] = reinterpret_cast<const uint32_t*>(g_slots)[i];
+    for (uint32_t i = threadIdx.x; i < V; i += NT) sp.arrivals[i] = 0u;
+    for (uint32_t i = threadIdx.x; i < g.W; i += NT) {
+        sp.act[i] = g.act[i];
+        sp.touch[i] = sp.dep[i] = 0u;
+        sp.tidy[i] = g.tidy[i];
+    }
+    if (threadIdx.x == 0) {
+        *contended = *g_contended;
+        for (uint32_t i = VK & ~3u; i < VK; i++) slots[i] = g_slots[i];  // a last, partial word
+    }
+    const RefRange R = ref_range(sm, sp.cw);
+    int32_t* const s_delta = reinterpret_cast<int32_t*>(sm + ref_range_words(sp.cw));
+    float* const s_P = reinterpret_cast<float*>(s_delta + p.S1 + 2);
+    uint32_t* const s_tab = reinterpret_cast<uint32_t*>(s_P + (stage_P ? p.NR * p.NR * p.S1 : 0u));
+    ref_stage_P(p, s_P, stage_P);
+    for (uint32_t s = threadIdx.x; s < p.S1 + 2; s += NT) s_delta[s] = 0;
+    RefTables T{};
+    if (rows) T = ref_stage_tables(p, sp, s_tab);
+    int32_t* const row = reinterpret_cast<int32_t*>(s_tab + ref_table_words(p.S1, p.R, sp.UW)) + threadIdx.x * p.S1;
+    __syncthreads();
     for (uint32_t k = 0; k < n; k++) {
-        ref_sp_list_act_body(sp);
+        const uint32_t itime = __ldg(itimes + step0 + k);
+        ref_sp_directions_body<KT, NT>(p, sp, slots, occ, itime, diag, contended, R, stage_P ? s_P : p.P);
         __syncthreads();
-        ref_sp_directions_body(p, sp, slots, occ, itimes, step0 + k, diag, contended, stage_P);
+        const uint32_t full = ref_word(contended);
+        if (full) ref_sp_serial_body(p, sp, slots, occ, conc, diag, s_words);
+        else ref_sp_gather_body<KT, NT>(p, sp, slots, occ, conc, R);
         __syncthreads();
-        ref_sp_list_touch_body(sp);
-        __syncthreads();
-        ref_sp_gather_body(p, sp, slots, occ, conc, contended);
-        __syncthreads();
-        ref_sp_serial_body(p, sp, slots, occ, conc, diag, contended);
-        __syncthreads();
+        if (full && threadIdx.x == 0) *contended = 0u;  // every thread has read it
         const uint32_t dense = ((k == 0u && dense_first) || dense_always) ? 1u : 0u;
-        ref_sp_cme_body(p, sp, slots, occ, conc, itimes, step0 + k, dense, stat, diag, contended, rows);
+        ref_sp_cme_body<KT, NT>(p, sp, slots, occ, conc, itime, dense, R, T, s_delta, row, rows);
         __syncthreads();
-        sp.c ^= 1u;
+    }
+    for (uint32_t i = threadIdx.x; i < VK / 4u; i += NT)
+        reinterpret_cast<uint32_t*>(g_slots)[i] = reinterpret_cast<const uint32_t*>(slots)[i];
+    for (uint32_t i = (VK & ~3u) + threadIdx.x; i < VK; i += NT) g_slots[i] = slots[i];
+    for (uint32_t i = threadIdx.x; i < g.W; i += NT) {
+        g.act[i] = sp.act[i];
+        g.tidy[i] = sp.tidy[i];
+    }
+    if (threadIdx.x == 0) *g_contended = 0u;
+    ref_flush_block(p, s_delta, stat, diag);
+}
+
+// act and tidy of a freshly uploaded lattice, a warp per word (no voxel is tidy without `rows`).
+__global__ void __launch_bounds__(256) ref_sp_build(RefParams p, RefSparse sp, const uint8_t* slots, const uint32_t* occ,
+                                                    const int32_t* conc, uint32_t rows) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t i = blockIdx.x * 8u + (threadIdx.x >> 5); i < sp.W; i += gridDim.x * 8u) {
+        const uint64_t v = (uint64_t)i * 32u + lane;
+        bool keep = false, tidy = false;
+        if (v < p.V) {
+            const RefSlots sl = rs_load(slots + v * p.K, p.K);
+            const RefMask full = rs_full(sl);
+            tidy = rows != 0u && occ[v] == rm_count(full);
+            keep = occ[v] != 0u || rm_any(full);
+            for (uint32_t s = 1; s < p.S1; s++) {
+                int32_t n = 0;
+                for (RefMask f = full; rm_any(f); rm_drop(f)) n += rs_get(sl, rm_first(f)) == s;
+                const int32_t c = conc[v * p.S1 + s];
+                keep |= c != 0;
+                tidy &= c == n;
+            }
+            for (RefMask f = full; rm_any(f); rm_drop(f)) tidy &= rs_get(sl, rm_first(f)) < p.S1;
+        }
+        const uint32_t k = __ballot_sync(0xffffffffu, keep), t = __ballot_sync(0xffffffffu, tidy);
+        if (lane == 0u) {
+            sp.act[i] = k;
+            sp.tidy[i] = t;
+        }
     }
 }
 
-// Act bitmap c of a freshly uploaded lattice.
-__global__ void ref_sp_build_act(RefParams p, RefSparse sp, const uint8_t* __restrict__ slots,
-                                 const uint32_t* __restrict__ occ, const int32_t* __restrict__ conc) {
-    for (uint32_t v = grid_tid(); v < (uint32_t)p.V; v += grid_threads()) {
-        bool keep = occ[v] != 0u;
-        for (uint32_t s = 0; s < p.K && !keep; s++) keep |= slots[(size_t)v * p.K + s] != 0u;
-        for (uint32_t s = 1; s < p.S1 && !keep; s++) keep |= conc[(size_t)v * p.S1 + s] != 0;
-        if (keep) set_bit(act_cur(sp), v);
+// The occupancy and the concentration rows of the tidy voxels, from their slots (frames have run: their
+// first reaction pass has set every row's entry 0).
+__global__ void __launch_bounds__(256) ref_write_rows(RefParams p, RefSparse sp, const uint8_t* slots, uint32_t* occ,
+                                                      int32_t* conc) {
+    for (uint64_t v = (uint64_t)blockIdx.x * 256u + threadIdx.x; v < p.V; v += (uint64_t)gridDim.x * 256u) {
+        if (!bit_of(sp.tidy, (uint32_t)v)) continue;
+        const RefSlots sl = rs_load(slots + v * p.K, p.K);
+        RefMask full = rs_full(sl);
+        int32_t* const c = conc + v * p.S1;
+        occ[v] = rm_count(full);
+        c[0] = 1;
+        for (uint32_t s = 1; s < p.S1; s++) c[s] = 0;
+        for (; rm_any(full); rm_drop(full)) c[rs_get(sl, rm_first(full))]++;
+    }
+}
+
+// Voxels whose six neighbours lie in the lattice and share their region, a warp per word.
+__global__ void __launch_bounds__(256) ref_same_regions(RefParams p, uint32_t* same, uint32_t W) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t i = blockIdx.x * 8u + (threadIdx.x >> 5); i < W; i += gridDim.x * 8u) {
+        const uint64_t v = (uint64_t)i * 32u + lane;
+        bool is = false;
+        if (v < p.V) {
+            uint32_t x, y, z;
+            ref_coords(p, (uint32_t)v, x, y, z);
+            if (x > 0u && x < p.X - 1u && y > 0u && y < p.Y - 1u && z > 0u && z < p.Z - 1u) {
+                const uint8_t* r = p.regions + v;
+                const uint8_t q = *r;
+                is = r[-(int64_t)p.YZ] == q && r[p.YZ] == q && r[-(int64_t)p.Z] == q && r[p.Z] == q && r[-1] == q && r[1] == q;
+            }
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, is);
+        if (lane == 0u) same[i] = m;
+    }
+}
+
+// RefSparse::fire1: the propensity sum of a voxel whose only particle is q, by the operations of the
+// reaction pass in their order.
+__global__ void ref_fire_table(RefParams p, float* fire1) {
+    for (uint32_t q = threadIdx.x; q < p.S1; q += blockDim.x) {
+        float total = 0.0f;
+        for (uint32_t r = 1; r <= p.R; r++) {
+            uint32_t prod = 1u;
+            for (uint32_t j = 0; j < 3; j++) {
+                const uint32_t a = p.reactants[r * 3 + j];
+                prod *= (a == 0u || a == q) ? 1u : 0u;
+            }
+            total = __fadd_rn(total, __fmul_rn(p.rates[r], __int2float_rn((int32_t)prod)));
+        }
+        fire1[q] = __fsub_rn(1.0f, d_expf(__fmul_rn(-total, p.tau)));
     }
 }
 
 // ------------------------------------------------------------------ host side
 
+// Bytes of the one-block form's state.
+static size_t ref_state_bytes(const RefParams& p) {
+    const size_t VKa = ((size_t)(p.V * p.K) + 15u) & ~(size_t)15u, W = ((size_t)p.V + 31u) / 32u;
+    return 3 * VKa + 4 * (size_t)p.V + 16 * W;
+}
+static bool ref_one_block(const DeviceRef* d) { return d->one_block; }
+
 static RefSparse ref_sparse(DeviceRef* d) {
     RefSparse sp{};
-    for (int b = 0; b < 2; b++) sp.act_bm[b] = d->act_bm[b].p;
-    sp.touch_bm = d->touch_bm.p;
-    sp.dep_bm = d->dep_bm.p;
-    sp.act_list = d->act_list.p;
-    sp.touch_list = d->touch_list.p;
-    sp.union_list = d->union_list.p;
-    sp.cnt = d->cnt.p;
+    sp.act = d->act_bm.p;
+    sp.touch = d->touch_bm.p;
+    sp.dep = d->dep_bm.p;
+    sp.tidy = d->tidy_bm.p;
+    sp.same = d->same_bm.p;
     sp.arrivals = d->arrivals.p;
     sp.dirs = d->dirs.p;
     sp.snap = d->snap.p;
+    sp.uses = d->uses.p;
+    sp.fire1 = d->fire1.p;
     sp.W = (uint32_t)d->touch_bm.n;
-    sp.c = d->par;
+    // a range per block: four blocks per SM where the lattice has the words for it (us per frame with two /
+    // four / eight: 64^3 with 22,000 particles 19.7 / 18.5 / 21.9, 100^3 with 40,000 29.9 / 24.2 / 29.3), and no
+    // more words than a block has threads
+    sp.cw = ref_one_block(d) ? sp.W : std::min<uint32_t>(REF_NT, std::max<uint32_t>(1u, sp.W / (4u * (uint32_t)d->sms)));
+    sp.UW = d->p.R / 32u + 1u;
+    sp.finite = d->finite ? 1u : 0u;
     return sp;
+}
+
+// Shared memory (bytes) of the passes in blocks of nt threads, with ranges of cw words: the range, the
+// S1 + 2 counters and, when they fit beside them in `limit` (rows), the reaction tables and a row per
+// thread; the directions pass stages the probability table when it takes at most 16 KB.
+static size_t ref_cme_smem(const RefParams& p, const RefSparse& sp, int nt, size_t other, size_t limit, uint32_t& rows) {
+    const size_t base = (ref_range_words(sp.cw) + p.S1 + 2) * 4 + other;
+    const size_t all = base + (ref_table_words(p.S1, p.R, sp.UW) + (size_t)nt * p.S1) * 4;
+    rows = all <= limit ? 1u : 0u;
+    return rows ? all : base;
+}
+static size_t ref_P_smem(const RefParams& p, uint32_t& stage_P) {
+    const size_t smem_P = (size_t)p.NR * p.NR * p.S1 * sizeof(float);
+    stage_P = smem_P <= 16u * 1024u ? 1u : 0u;
+    return stage_P ? smem_P : 0u;
+}
+
+// Shared memory of the one-block form, or 0 when it does not fit; other: the bytes before its state.
+static size_t ref_block_smem(const DeviceRef* d, const RefSparse& sp, uint32_t& stage_P, uint32_t& rows, uint32_t& other) {
+    const size_t P = ref_P_smem(d->p, stage_P);
+    const size_t state = ref_state_bytes(d->p) + 16u, most = (size_t)d->smem_optin - 4096u;
+    if (state >= most) return 0u;
+    other = (uint32_t)((ref_cme_smem(d->p, sp, REF_BLOCK_THREADS, P, most - state, rows) + 15u) & ~(size_t)15u);
+    const size_t all = other + state;
+    return all <= most ? all : 0u;
+}
+
+// Whether the reaction pass runs on shared-memory rows (tidy voxels need them).
+static uint32_t ref_rows(const DeviceRef* d, const RefSparse& sp) {
+    uint32_t rows = 0, stage_P = 0, other = 0;
+    if (ref_one_block(d)) ref_block_smem(d, sp, stage_P, rows, other);
+    else ref_cme_smem(d->p, sp, REF_NT, 0, REF_SMEM, rows);
+    return rows;
+}
+
+template <int KT>
+static void ref_block_attr(int bytes) {
+    CS_CUDA(cudaFuncSetAttribute(ref_sp_frames_block<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
+// Chooses the form for a lattice of `particles` particles.
+static void ref_choose_form(DeviceRef* d, uint64_t particles) {
+    d->one_block = d->p.V <= REF_BLOCK_MAX_VOXELS && particles <= REF_BLOCK_MAX_PARTICLES;
+    if (!d->one_block) return;
+    uint32_t rows = 0, stage_P = 0, other = 0;
+    if (!ref_block_smem(d, ref_sparse(d), stage_P, rows, other) || !rows) {
+        d->one_block = false;
+        return;
+    }
+    const int most = d->smem_optin - 4096;
+    if (d->p.K == 16u) ref_block_attr<16>(most);
+    else if (d->p.K == 8u) ref_block_attr<8>(most);
+    else ref_block_attr<0>(most);
 }
 
 static void ref_bind(DeviceRef* d) {
@@ -1043,18 +1437,15 @@ DeviceRef* ref_create(const Model& m, int device) {
     d->dirs.alloc(VK);
     d->snap.alloc(VK);
     const uint64_t W = (m.V + 31) / 32;
-    for (int b = 0; b < 2; b++) d->act_bm[b].alloc(W);
+    d->act_bm.alloc(W);
     d->touch_bm.alloc(W);
     d->dep_bm.alloc(W);
-    d->act_list.alloc(m.V);
-    d->touch_list.alloc(m.V);
-    d->union_list.alloc(m.V);
-    d->cnt.alloc(3);
+    d->tidy_bm.alloc(W);
+    d->same_bm.alloc(W);
     d->arrivals.alloc(m.V);
     CS_CUDA(cudaMemset(d->arrivals.p, 0, m.V * 4));
-    int sms = 1;
-    CS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    d->grid = sms * 8;
+    CS_CUDA(cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, device));
+    CS_CUDA(cudaDeviceGetAttribute(&d->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     for (uint32_t r = 1; r <= m.n_reactions; r++)
         if (m.reactants[r * 3] == 0u && m.reactants[r * 3 + 1] == 0u && m.reactants[r * 3 + 2] == 0u)
             d->dense_always = true;
@@ -1078,6 +1469,19 @@ DeviceRef* ref_create(const Model& m, int device) {
     CS_CUDA(cudaMemcpy(d->reactants.p, m.reactants.data(), m.reactants.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     CS_CUDA(cudaMemset(d->diag.p, 0, DIAG_N * sizeof(uint32_t)));
     CS_CUDA(cudaMemset(d->flag.p, 0, sizeof(uint32_t)));
+    const uint32_t UW = p.R / 32u + 1u;
+    std::vector<uint32_t> uses((size_t)p.S1 * UW, 0u);
+    for (uint32_t r = 1; r <= p.R; r++) {
+        d->finite = d->finite && std::isfinite(m.rates[r]);
+        for (uint32_t j = 0; j < 3; j++) uses[(size_t)m.reactants[r * 3 + j] * UW + r / 32u] |= 1u << (r & 31u);
+    }
+    d->uses.alloc(uses.size());
+    CS_CUDA(cudaMemcpy(d->uses.p, uses.data(), uses.size() * 4, cudaMemcpyHostToDevice));
+    d->fire1.alloc(p.S1);
+    ref_fire_table<<<1, 256, 0, d->stream>>>(p, d->fire1.p);
+    CS_LAUNCH_CHECK();
+    ref_same_regions<<<2048, 256, 0, d->stream>>>(p, d->same_bm.p, (uint32_t)W);
+    CS_LAUNCH_CHECK();
     std::vector<int32_t> conc = m.concentrations();
     ref_set_lattice(d.get(), m.slots.data(), m.occupancy.data(), conc.data());
     return d.release();
@@ -1102,18 +1506,19 @@ void ref_set_lattice(DeviceRef* d, const uint32_t* slots, const uint32_t* occ, c
     CS_CUDA(cudaMemcpy(d->slots.p, s8.data(), VK, cudaMemcpyHostToDevice));
     CS_CUDA(cudaMemcpy(d->occ.p, occ, d->p.V * sizeof(uint32_t), cudaMemcpyHostToDevice));
     CS_CUDA(cudaMemcpy(d->conc.p, conc, VS * sizeof(int32_t), cudaMemcpyHostToDevice));
-    // the sparse passes start from the act list of the new lattice and empty
-    // touch lists and bitmaps; its first reaction pass visits every voxel
-    // (conc[v][0] = 1, compaction)
+    // the sparse passes start from the act bitmap of the new lattice and empty touch and departure
+    // bitmaps; its first reaction pass visits every voxel (conc[v][0] = 1, compaction)
     const size_t wb = d->touch_bm.bytes();
-    for (int b = 0; b < 2; b++) CS_CUDA(cudaMemset(d->act_bm[b].p, 0, wb));
     CS_CUDA(cudaMemset(d->touch_bm.p, 0, wb));
     CS_CUDA(cudaMemset(d->dep_bm.p, 0, wb));
-    CS_CUDA(cudaMemset(d->cnt.p, 0, d->cnt.bytes()));
     CS_CUDA(cudaMemset(d->arrivals.p, 0, d->arrivals.bytes()));
-    d->par = 0;
-    ref_sp_build_act<<<d->grid, 256, 0, d->stream>>>(d->p, ref_sparse(d), d->slots.p, d->occ.p, d->conc.p);
+    uint64_t particles = 0;
+    for (uint64_t i = 0; i < VK; i++) particles += s8[i] != 0u;
+    ref_choose_form(d, particles);
+    const RefSparse sp = ref_sparse(d);
+    ref_sp_build<<<d->sms * 8, 256, 0, d->stream>>>(d->p, sp, d->slots.p, d->occ.p, d->conc.p, ref_rows(d, sp));
     CS_LAUNCH_CHECK();
+    d->rows_stale = false;
     CS_CUDA(cudaStreamSynchronize(d->stream));
     d->dense_next = true;
     // create_statistics, src/simulation.rs:361-388: the counts restart from the sum of the concentrations
@@ -1158,6 +1563,11 @@ void ref_render_view(DeviceRef* d, int32_t view, int32_t slice_axis, uint32_t sl
 
 void ref_get_lattice(DeviceRef* d, uint32_t* slots, uint32_t* occ, int32_t* conc) {
     DeviceGuard g(d->device);
+    if ((occ || conc) && d->rows_stale) {
+        ref_write_rows<<<d->sms * 8, 256, 0, d->stream>>>(d->p, ref_sparse(d), d->slots.p, d->occ.p, d->conc.p);
+        CS_LAUNCH_CHECK();
+        d->rows_stale = false;
+    }
     CS_CUDA(cudaStreamSynchronize(d->stream));
     uint64_t VK = d->p.V * d->p.K, VS = d->p.V * d->p.S1;
     if (slots) {
@@ -1169,8 +1579,7 @@ void ref_get_lattice(DeviceRef* d, uint32_t* slots, uint32_t* occ, int32_t* conc
     if (conc) CS_CUDA(cudaMemcpy(conc, d->conc.p, VS * sizeof(int32_t), cudaMemcpyDeviceToHost));
 }
 
-// Enqueues the sparse passes of one frame reading itimes[k].
-// A launch with programmatic stream serialization (see ref_pdl_start).
+// A launch with programmatic stream serialization (see ref_wait_previous).
 template <typename... KArgs, typename... Args>
 static void ref_launch(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg{};
@@ -1186,58 +1595,51 @@ static void ref_launch(void (*kernel)(KArgs...), int grid, int block, size_t sme
     CS_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
-// Shared memory of the reaction pass in blocks of tb threads: it stages the tables and one
-// concentration row per thread when they fit in the default 48 KB (rows = 1).
-static size_t ref_cme_smem(const RefParams& p, int tb, uint32_t& rows) {
-    const size_t smem_rows =
-        ((size_t)p.S1 + 2 + 4 * ((size_t)p.R + 1) + ((size_t)p.R + 1) * p.S1 + (size_t)tb * p.S1) * 4;
-    rows = smem_rows <= 48u * 1024u ? 1u : 0u;
-    return rows ? smem_rows : (p.S1 + 2) * sizeof(int32_t);
-}
-
-// The directions pass stages the probability table in shared memory when it takes at most 16 KB.
-static size_t ref_dir_smem(const RefParams& p, uint32_t& stage_P) {
-    const size_t smem_P = (size_t)p.NR * p.NR * p.S1 * sizeof(float);
-    stage_P = smem_P <= 16u * 1024u ? 1u : 0u;
-    return stage_P ? smem_P : 0u;
-}
-
-static bool ref_one_block(const DeviceRef* d) { return d->p.V <= REF_BLOCK_MAX_VOXELS; }
-
 // Frames k0 .. k0 + n - 1 of the call (itimes[k]) in one launch of the one-block form.
+template <int KT>
+static void ref_enqueue_block_k(DeviceRef* d, uint32_t k0, uint32_t n) {
+    const RefParams& p = d->p;
+    const RefSparse sp = ref_sparse(d);
+    uint32_t rows = 0, stage_P = 0, other = 0;
+    const size_t smem = ref_block_smem(d, sp, stage_P, rows, other);
+    ref_sp_frames_block<KT><<<1, REF_BLOCK_THREADS, smem, d->stream>>>(
+        p, sp, d->slots.p, d->occ.p, d->conc.p, (const uint32_t*)d->itimes.p, k0, n, d->dense_next ? 1u : 0u,
+        d->dense_always ? 1u : 0u, d->stat.p, d->diag.p, d->flag.p, stage_P, rows, other);
+    CS_LAUNCH_CHECK();
+}
+
 static void ref_enqueue_block(DeviceRef* d, uint32_t k0, uint32_t n) {
     if (n == 0) return;
+    if (d->p.K == 16u) ref_enqueue_block_k<16>(d, k0, n);
+    else if (d->p.K == 8u) ref_enqueue_block_k<8>(d, k0, n);
+    else ref_enqueue_block_k<0>(d, k0, n);
+    d->dense_next = false;
+    d->rows_stale = true;
+}
+
+template <int KT>
+static void ref_enqueue_frame_k(DeviceRef* d, uint32_t k) {
     const RefParams& p = d->p;
     const RefSparse sp = ref_sparse(d);
     uint32_t rows = 0, stage_P = 0;
-    const size_t smem = std::max(ref_cme_smem(p, REF_BLOCK_THREADS, rows), ref_dir_smem(p, stage_P));
-    ref_sp_frames_block<<<1, REF_BLOCK_THREADS, smem, d->stream>>>(
-        p, sp, d->slots.p, d->occ.p, d->conc.p, (const uint32_t*)d->itimes.p, k0, n, d->dense_next ? 1u : 0u,
-        d->dense_always ? 1u : 0u, d->stat.p, d->diag.p, d->flag.p, stage_P, rows);
-    CS_LAUNCH_CHECK();
-    d->dense_next = false;
-    d->par ^= n & 1u;
+    const size_t range = ref_range_words(sp.cw) * 4, P = ref_P_smem(p, stage_P);
+    const size_t smem = ref_cme_smem(p, sp, REF_NT, 0, REF_SMEM, rows);
+    const int grid = (int)std::min<uint32_t>((sp.W + sp.cw - 1u) / sp.cw, 16u * (uint32_t)d->sms);
+    const uint32_t dense = (d->dense_next || d->dense_always) ? 1u : 0u;
+    ref_launch(ref_sp_directions<KT>, grid, REF_NT, range + P, d->stream, p, sp, (const uint8_t*)d->slots.p,
+               (const uint32_t*)d->occ.p, (const uint32_t*)d->itimes.p, k, d->diag.p, d->flag.p, stage_P);
+    ref_launch(ref_sp_move<KT>, grid, REF_NT, range, d->stream, p, sp, d->slots.p, d->occ.p, d->conc.p, d->diag.p,
+               (const uint32_t*)d->flag.p);
+    ref_launch(ref_sp_cme<KT>, grid, REF_NT, smem, d->stream, p, sp, d->slots.p, d->occ.p, d->conc.p,
+               (const uint32_t*)d->itimes.p, k, dense, d->stat.p, d->diag.p, d->flag.p, rows);
 }
 
 static void ref_enqueue_frame(DeviceRef* d, uint32_t k) {
-    const RefParams& p = d->p;
-    const RefSparse sp = ref_sparse(d);
-    const int TB = 256;
-    uint32_t rows = 0, stage_P = 0;
-    const size_t smem = ref_cme_smem(p, TB, rows);
-    ref_launch(ref_sp_list_act, d->grid, TB, 0, d->stream, sp);
-    const size_t smem_P = ref_dir_smem(p, stage_P);
-    ref_launch(ref_sp_directions, d->grid, TB, smem_P, d->stream, p, sp, (const uint8_t*)d->slots.p,
-               (const uint32_t*)d->occ.p, (const uint32_t*)d->itimes.p, k, d->diag.p, d->flag.p, stage_P);
-    ref_launch(ref_sp_list_touch, d->grid, TB, 0, d->stream, sp);
-    ref_launch(ref_sp_gather, d->grid, TB, 0, d->stream, p, sp, d->slots.p, d->occ.p, d->conc.p, d->flag.p);
-    ref_launch(ref_sp_serial, 1, 1024, 0, d->stream, p, sp, d->slots.p, d->occ.p, d->conc.p, d->diag.p, d->flag.p);
-    const uint32_t dense = (d->dense_next || d->dense_always) ? 1u : 0u;
-    ref_launch(ref_sp_cme, d->grid, TB, smem, d->stream, p, sp, d->slots.p, d->occ.p, d->conc.p,
-               (const uint32_t*)d->itimes.p, k, dense, d->stat.p, d->diag.p, d->flag.p, rows);
-    CS_LAUNCH_CHECK();
+    if (d->p.K == 16u) ref_enqueue_frame_k<16>(d, k);
+    else if (d->p.K == 8u) ref_enqueue_frame_k<8>(d, k);
+    else ref_enqueue_frame_k<0>(d, k);
     d->dense_next = false;
-    d->par ^= 1u;
+    d->rows_stale = true;
 }
 
 static void ref_enqueue(DeviceRef* d, uint32_t n) {
