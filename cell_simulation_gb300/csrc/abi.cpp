@@ -344,8 +344,9 @@ cs_status cs_set_lattice(cs_sim* sim, const uint32_t* slots, const uint32_t* occ
         Model& m = sim->model;
         uint32_t s1 = m.n_species + 1;
         std::vector<uint32_t> occ(m.V);
-        for (uint64_t i = 0; i < m.V * m.K; i++)
-            if (slots[i] > m.n_species) throw Error(CS_ERR_INVALID_ARG, "slot species out of range");
+        uint32_t most = 0;  // no branch per slot: the loop vectorises
+        for (uint64_t i = 0; i < m.V * m.K; i++) most = slots[i] > most ? slots[i] : most;
+        if (most > m.n_species) throw Error(CS_ERR_INVALID_ARG, "slot species out of range");
         if (occupancy) {
             std::memcpy(occ.data(), occupancy, m.V * sizeof(uint32_t));
         } else {
@@ -356,7 +357,7 @@ cs_status cs_set_lattice(cs_sim* sim, const uint32_t* slots, const uint32_t* occ
             }
         }
         m.slots.assign(slots, slots + m.V * m.K);
-        m.occupancy = occ;
+        m.occupancy = std::move(occ);
         if (concentrations) {
             m.conc.assign(concentrations, concentrations + m.V * s1);
             m.conc_explicit = true;
