@@ -544,8 +544,8 @@ void lists_set_attrs(int device) {
     int optin = 0;
     CS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     void* fns[] = {reinterpret_cast<void*>(&list_frames_kernel<8, 256>), reinterpret_cast<void*>(&list_frames_kernel<8, 512>),
-                   reinterpret_cast<void*>(&list_frames_kernel<16, 256>),
-                   reinterpret_cast<void*>(&list_frames_kernel<16, 512>)};
+                   reinterpret_cast<void*>(&list_frames_kernel<8, 768>), reinterpret_cast<void*>(&list_frames_kernel<16, 256>),
+                   reinterpret_cast<void*>(&list_frames_kernel<16, 512>), reinterpret_cast<void*>(&list_frames_kernel<16, 768>)};
     for (void* fn : fns) {
         CS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         CS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
@@ -555,10 +555,9 @@ void lists_set_attrs(int device) {
 void lists_launch(int K, int threads, const ListParams& P, uint32_t grid, cudaStream_t s) {
     if (grid == 0 || P.n_frames == 0) return;
     const size_t smem = lists_smem(K, P.cap, P.thr_words);
-    if (K == 16 && threads == 512) list_frames_kernel<16, 512><<<grid, 512, smem, s>>>(P);
-    else if (K == 16) list_frames_kernel<16, 256><<<grid, 256, smem, s>>>(P);
-    else if (threads == 512) list_frames_kernel<8, 512><<<grid, 512, smem, s>>>(P);
-    else list_frames_kernel<8, 256><<<grid, 256, smem, s>>>(P);
+    auto run = [&](auto kernel) { kernel<<<grid, threads, smem, s>>>(P); };
+    if (K == 16) run(threads == 768 ? list_frames_kernel<16, 768> : threads == 512 ? list_frames_kernel<16, 512> : list_frames_kernel<16, 256>);
+    else run(threads == 768 ? list_frames_kernel<8, 768> : threads == 512 ? list_frames_kernel<8, 512> : list_frames_kernel<8, 256>);
     CS_LAUNCH_CHECK();
 }
 

@@ -1736,8 +1736,10 @@ static bool run_lists(DeviceProd* d, uint32_t n, bool batched) {
     ListParams P = lists_params(d);
     P.frame0 = (uint32_t)d->next_frame;
     P.n_frames = n;
-    // 512 threads where SMs have at most one block anyway: fewer rounds of a sweep's entries
-    const int threads = d->n_rep <= (uint32_t)d->num_sms && d->p_max > 128 ? 512 : 256;
+    // more threads where SMs have at most one block anyway: fewer rounds of a sweep's entries and more warps
+    // for the SSAs, against dearer barriers (us per frame with 512 / 768 threads, 96 replicates of the 12-species
+    // network on 12 .. 24 cubed voxels: 300 particles 11.5 / 11.9, 450 15.7 / 14.0, 600 20.0 / 19.1, 780 25.1 / 22.9)
+    const int threads = d->n_rep > (uint32_t)d->num_sms || d->p_max <= 128 ? 256 : d->p_max <= 350 ? 512 : 768;
     if (batched) {
         lists_launch((int)d->K, threads, P, d->n_rep, d->stream);
     } else {

@@ -33,8 +33,8 @@
 // What bounds it: instructions and shared-memory round trips of one block per SM;
 // a frame is six dependent steps and the SSA (about 4k cycles for a sweep's first
 // step, 2.5k - 3.5k for its second, 1k - 7k for the SSA on the ensemble below), and
-// no DRAM traffic remains.  512 threads where an SM has one block anyway, else 256
-// so that two or three share an SM.  us per frame, fused sweep stream / lists: the
+// no DRAM traffic remains.  512 or 768 threads where an SM has one block anyway,
+// else 256 so that two or three share an SM.  us per frame, fused sweep stream / lists: the
 // 512 replicates above 336 / 38; 96 replicates of the stiff network with 600
 // particles on 12..24 cubed voxels 43.6 / 22.7.
 #pragma once

@@ -64,6 +64,14 @@ def test_word_edges_match_oracle(orc, form, K, res):
     check(orc, mk, 12, 91, form(K))
 
 
+@pytest.mark.parametrize("K", [8, 16])
+@pytest.mark.parametrize("particles", [128, 129, 350, 351, 600])
+def test_threads_of_a_list_block(orc, K, particles):
+    """Both sides of the lines between 256, 512 and 768 threads."""
+    check(orc, lambda: one_region((11, 13, 17), K, (particles - particles // 2, particles // 2, 0), (300.0, 60.0, 0.0)),
+          12, 57, lists(K))
+
+
 @pytest.mark.parametrize("form", [lists, in_place])
 @pytest.mark.parametrize("K", [8, 16])
 def test_regions_match_oracle(orc, form, K):
