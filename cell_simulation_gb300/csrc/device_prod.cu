@@ -1734,18 +1734,21 @@ static bool run_lists(DeviceProd* d, uint32_t n, bool batched) {
         lists_pack((int)d->K, lists_params(d), d->n_rep, max_rep_voxels(d), d->stream);
     }
     ListParams P = lists_params(d);
-    P.frame0 = (uint32_t)d->next_frame;
-    P.n_frames = n;
     // more threads where SMs have at most one block anyway: fewer rounds of a sweep's entries and more warps
     // for the SSAs, against dearer barriers (us per frame with 512 / 768 threads, 96 replicates of the 12-species
     // network on 12 .. 24 cubed voxels: 300 particles 11.5 / 11.9, 450 15.7 / 14.0, 600 20.0 / 19.1, 780 25.1 / 22.9)
     const int threads = d->n_rep > (uint32_t)d->num_sms || d->p_max <= 128 ? 256 : d->p_max <= 350 ? 512 : 768;
-    if (batched) {
-        lists_launch((int)d->K, threads, P, d->n_rep, d->stream);
-    } else {
-        for (uint32_t r = 0; r < d->n_rep; r++) {
-            P.rep0 = r;
-            lists_launch((int)d->K, threads, P, 1, d->stream);
+    for (uint32_t k = 0; k < n; k += P.n_frames) {
+        P.frame0 = (uint32_t)(d->next_frame + k);
+        P.n_frames = std::min(n - k, LIST_MAX_FRAMES);
+        if (batched) {
+            P.rep0 = 0;
+            lists_launch((int)d->K, threads, P, d->n_rep, d->stream);
+        } else {
+            for (uint32_t r = 0; r < d->n_rep; r++) {
+                P.rep0 = r;
+                lists_launch((int)d->K, threads, P, 1, d->stream);
+            }
         }
     }
     d->next_frame += n;

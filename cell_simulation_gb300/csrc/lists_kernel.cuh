@@ -48,6 +48,10 @@ namespace cellsim {
 
 constexpr uint32_t LIST_DENSE = 0xFFFFFFFFu;  // ListParams::n of a replicate whose state is in the slots
 constexpr uint32_t LIST_MAX_EDGE = 1024;
+// Most frames of a launch.  An entry's Philox block is valid in the frame that its 16-bit tag names, and an
+// emptied entry keeps its tag for as long as the list is not compacted: a launch, which starts every tag
+// afresh, must end before the tags come round (65,536 frames).
+constexpr uint32_t LIST_MAX_FRAMES = 32768;
 
 struct ListParams {
     ProdTables T;
@@ -62,7 +66,7 @@ struct ListParams {
     uint32_t cap;               // entries per replicate, in global and in shared memory
     unsigned long long* counts;
     uint32_t* diag;
-    uint32_t rep0, frame0, n_frames;
+    uint32_t rep0, frame0, n_frames;  // n_frames: at most LIST_MAX_FRAMES
     uint32_t* step_out;         // the next frame's number goes here
     uint32_t* host_flag;        // host-visible word: set when a replicate went LIST_DENSE
     uint32_t thr_words;         // words of the threshold table staged in shared memory (0: read from global)
