@@ -481,6 +481,14 @@ cs_status cs_debug_stall_group(cs_sim* sim, uint32_t group) {
     });
 }
 
+cs_status cs_debug_refuse_tiling(cs_sim* sim, int32_t index, cs_status status) {
+    return guarded([&] {
+        need(sim, "sim");
+        if (!sim->prod) throw Error(CS_ERR_STATE, "cs_debug_refuse_tiling needs cs_prepare_for_gpu(CS_RNG_PHILOX)");
+        prod_debug_refuse_tiling(sim->prod.get(), index, status);
+    });
+}
+
 cs_status cs_step_timed(cs_sim* sim, uint32_t n_steps, const uint32_t* itimes, float* ms) {
     return guarded([&] {
         need(sim, "sim");

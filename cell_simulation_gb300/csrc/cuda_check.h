@@ -22,7 +22,12 @@
 
 namespace cellsim {
 
-// RAII device buffer.
+// The device has no room for an allocation; nothing else is wrong.
+struct OutOfMemory : Error {
+    using Error::Error;
+};
+
+// RAII device buffer (empty after a failed alloc).
 template <typename T>
 struct DevBuf {
     T* p = nullptr;
@@ -33,8 +38,16 @@ struct DevBuf {
     ~DevBuf() { reset(); }
     void alloc(size_t count) {
         reset();
+        if (count == 0) return;
+        const cudaError_t e = cudaMalloc((void**)&p, sizeof(T) * count);
+        if (e != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();  // or the next launch check would report it again
+            const std::string what = std::string("device allocation: ") + cudaGetErrorString(e);
+            if (e == cudaErrorMemoryAllocation) throw OutOfMemory(CS_ERR_CUDA, what);
+            throw Error(CS_ERR_CUDA, what);
+        }
         n = count;
-        if (count) CS_CUDA(cudaMalloc((void**)&p, sizeof(T) * count));
     }
     void reset() {
         if (p) cudaFree(p);

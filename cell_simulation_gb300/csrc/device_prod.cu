@@ -207,6 +207,8 @@ struct DeviceProd {
     DevBuf<uint32_t> nbr, done1, done2, frames_ctr;
     DevBuf<uint32_t> plane_order;  // the sorted position of each group in build (plane) order
     uint32_t frames_seq = 0;
+    int refuse_cfg = -1;                 // cs_debug_refuse_tiling: the variant that set_cfg refuses, and how
+    cs_status refuse_status = CS_ERR_LIMIT;
     uint32_t stall_group = 0xFFFFFFFFu;  // cs_debug_stall_group: the next multi-frame launch's stalled group
     std::vector<WordGroup> h_groups;
     bool groups_sorted = false;  // groups dealt heaviest first (sorted once per group build)
@@ -988,6 +990,7 @@ static void set_cfg(DeviceProd* d, int idx) {
     d->cfg_index = idx;
     try {
         build_items(d);
+        if (idx == d->refuse_cfg) throw Error(d->refuse_status, "variant refused by cs_debug_refuse_tiling");
     } catch (...) {
         d->cfg_index = prev;
         if (prev >= 0) build_items(d);
@@ -1225,6 +1228,10 @@ static void launch_stream_frames(DeviceProd* d, uint32_t n) {
 }
 
 void prod_debug_stall_group(DeviceProd* d, uint32_t group) { d->stall_group = group; }
+void prod_debug_refuse_tiling(DeviceProd* d, int cfg_index, cs_status status) {
+    d->refuse_cfg = cfg_index;
+    d->refuse_status = status;
+}
 
 static void launch_stream_frame(DeviceProd* d, const KernelCfg& cfg, const ProdParams& P, int rep, int parity) {
     const bool fused = stream_variant_fused(cfg.variant);
@@ -2239,44 +2246,69 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         d->ip_state = d->ip_valid = d->ls_state = d->slots_stale = false;
         d->frame_known = false;
     };
-    save(start);
-    size_t free_bytes = 0, all_bytes = 0;
-    CS_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
-    if (free_bytes > 4 * bytes) {  // else the trials start from the current state
-        prod_time_frames(d, kSettleFrames, frame0, batched);
-        save(settled);
-        frame0 += kSettleFrames;
-        from = &settled;
-        restore();
-    }
+    const int cfg0 = d->cfg_index;
+    const uint32_t seg0 = d->seg_len;
     const auto& c = all_cfgs();
     int best = -1;
     float best_t = 0.0f;
-    for (int i = 0; i < (int)c.size(); i++) {
-        if (c[i].K != (int)d->K) continue;
-        if (c[i].kind == KIND_STREAM && stream_variant_fused(c[i].variant) && !fused_fits(d)) continue;
-        if (c[i].kind == KIND_RESIDENT && !resident_fits(d)) continue;
-        if (c[i].kind == KIND_INPLACE && !inplace_fits(d)) continue;
-        if (c[i].kind == KIND_LISTS && !lists_cap(d)) continue;
-        d->seg_len = 0;
-        set_cfg(d, i);
-        prod_time_frames(d, 2, frame0, batched);  // warm-up: graph, bitmaps, caches
-        restore();
-        // the best of three trials, each after one untimed frame (the bitmap rebuild and the
-        // x-decisions that every restored state needs first): variants within a few percent of
-        // each other are then ranked by their steady frames, not by one noisy trial
-        float t = 0.0f;
-        for (int rep = 0; rep < 3; rep++) {
-            prod_time_frames(d, 1, frame0, batched);
-            const float r = prod_time_frames(d, frames, frame0 + 1, batched) / (float)frames;
+    save(start);
+    try {
+        size_t free_bytes = 0, all_bytes = 0;
+        CS_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
+        // room for the copy beside every variant's buffers (112 bytes per voxel of a bitmap word: the
+        // stream's records 96, the in-place form's decisions and species 13); else the trials start from
+        // the current state
+        if (free_bytes > 4 * bytes + 112ull * 32ull * d->occ_words) {
+            prod_time_frames(d, kSettleFrames, frame0, batched);
+            save(settled);
+            frame0 += kSettleFrames;
+            from = &settled;
             restore();
-            if (rep == 0 || r < t) t = r;
         }
-        if (best < 0 || t < best_t) { best = i; best_t = t; }
+        for (int i = 0; i < (int)c.size(); i++) {
+            if (c[i].K != (int)d->K) continue;
+            if (c[i].kind == KIND_STREAM && stream_variant_fused(c[i].variant) && !fused_fits(d)) continue;
+            if (c[i].kind == KIND_RESIDENT && !resident_fits(d)) continue;
+            if (c[i].kind == KIND_INPLACE && !inplace_fits(d)) continue;
+            if (c[i].kind == KIND_LISTS && !lists_cap(d)) continue;
+            d->seg_len = 0;
+            try {
+                set_cfg(d, i);
+            } catch (const OutOfMemory&) {
+                continue;  // no room for its buffers: no candidate
+            } catch (const Error& e) {
+                if (e.code != CS_ERR_LIMIT) throw;
+                continue;  // too large for its work lists: no candidate
+            }
+            prod_time_frames(d, 2, frame0, batched);  // warm-up: graph, bitmaps, caches
+            restore();
+            // the best of three trials, each after one untimed frame (the bitmap rebuild and the
+            // x-decisions that every restored state needs first): variants within a few percent of
+            // each other are then ranked by their steady frames, not by one noisy trial
+            float t = 0.0f;
+            for (int rep = 0; rep < 3; rep++) {
+                prod_time_frames(d, 1, frame0, batched);
+                const float r = prod_time_frames(d, frames, frame0 + 1, batched) / (float)frames;
+                restore();
+                if (rep == 0 || r < t) t = r;
+            }
+            if (best < 0 || t < best_t) { best = i; best_t = t; }
+        }
+        if (best < 0) throw Error(CS_ERR_LIMIT, "no step variant can be set up for this lattice");
+        set_cfg(d, best);
+        from = &start;
+        restore();
+    } catch (...) {
+        // the caller's state and variant, whatever failed (on a device error these calls fail too)
+        try {
+            from = &start;
+            restore();
+            d->seg_len = seg0;
+            set_cfg(d, cfg0);
+        } catch (...) {
+        }
+        throw;
     }
-    set_cfg(d, best);
-    from = &start;
-    restore();
     {
         std::lock_guard<std::mutex> lk(mu);
         cache[key] = {best, best_t};

@@ -354,6 +354,10 @@ class Simulation:
         """Test hook (cs_debug_stall_group): the next multi-frame launch's waits for `group` run out."""
         N.check(self._lib.cs_debug_stall_group(self._h, group))
 
+    def debug_refuse_tiling(self, index: int, status: int) -> None:
+        """Test hook (cs_debug_refuse_tiling): setting up variant `index` fails with `status` (-1: none)."""
+        N.check(self._lib.cs_debug_refuse_tiling(self._h, index, status))
+
     def _drain_stats(self) -> None:
         buf = (N.StatSampleC * 256)()
         names = None

@@ -226,6 +226,11 @@ cs_status cs_synchronize(cs_sim* sim);
  * out, the launch abandons its frames and the host reports the error.  No
  * reference counterpart. */
 cs_status cs_debug_stall_group(cs_sim* sim, uint32_t group);
+/* Test hook of what happens when a step variant cannot be set up: cs_set_tiling
+ * and the autotuner's trials of variant `index` fail with `status` from now on,
+ * after its work lists have been made (index -1: none fails).  No reference
+ * counterpart. */
+cs_status cs_debug_refuse_tiling(cs_sim* sim, int32_t index, cs_status status);
 
 /* ---------------- allocation-free reference-RNG frame ---------------- */
 /* Arguments of cs_ref_frame_noalloc.  Every pointer is a device pointer on
