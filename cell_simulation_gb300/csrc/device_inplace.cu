@@ -494,6 +494,10 @@ __global__ void __launch_bounds__(LINE_NT, 4) inplace_line_kernel(const __grid_c
         frame = AX == 0 ? *P.fa : *P.fb - 1u;
         if (blockIdx.x == 0 && tid == 0) *(AX == 0 ? P.fb : P.fa) = frame + 1u;
     }
+    if (P.from && (int32_t)(frame - P.from[ri]) < 0) {
+        cp_async_wait<0>();
+        return;
+    }
     const uint32_t lw = U.lw, pitch = 1u << lw, len = AX == 0 ? rd.X : rd.Y, T = len << lw;
     const uint32_t plane = rd.Y * rd.Wz;  // words of a plane
     // word idx: line position idx >> lw, column idx & (pitch - 1)
@@ -683,6 +687,15 @@ __global__ void __launch_bounds__(ROW_NT, 7) inplace_row_kernel(const __grid_con
     uint32_t frame = P.frame;  // of the sweep; the decisions are for `next`
     if (!P.explicit_frame) frame = P.decide_only ? *P.fa : *P.fa - 1u;
     const uint32_t next = P.decide_only ? frame : frame + 1u;
+    bool decide_only = P.decide_only != 0u;
+    if (P.from) {
+        const uint32_t from = P.from[ri];
+        if ((int32_t)(next - from) < 0) {
+            cp_async_wait<0>();
+            return;
+        }
+        decide_only |= (int32_t)(frame - from) < 0;
+    }
     uint2* const mv = P.mv[2] + gw0;
     uint8_t* const lat = P.lat + rd.base * K;
     uint8_t* const spec = P.spec + gw0 * 32u;
@@ -697,7 +710,7 @@ __global__ void __launch_bounds__(ROW_NT, 7) inplace_row_kernel(const __grid_con
             o[s] = u[s] = re[s] = 0u;
             t[s] = make_uint2(0u, 0u);
             if (idx < T) {
-                if (!P.decide_only) {
+                if (!decide_only) {
                     t[s] = mv[idx];
                     re[s] = P.react[gw0 + idx];
                 }
@@ -722,7 +735,7 @@ __global__ void __launch_bounds__(ROW_NT, 7) inplace_row_kernel(const __grid_con
         }
     }
     cp_async_wait<0>();
-    if (__syncthreads_or((int)(had != 0u || zero_order || P.resv_bits != nullptr) && !P.decide_only)) {
+    if (__syncthreads_or((int)(had != 0u || zero_order || P.resv_bits != nullptr) && !decide_only)) {
         uint32_t simple[NW], rest[NW], fill[NW], cnt = 0u;
 #pragma unroll
         for (int s = 0; s < NW; s++) {

@@ -93,71 +93,6 @@ __device__ __forceinline__ bool list_calm(const ProdTables& T, uint32_t ci, cons
                          T.a2 ? T.a2 + (size_t)ci * T.S1 * T.S1 : nullptr, T.tau);
 }
 
-// The rest of a step call over the whole lattice of a replicate (in P.lat, already written), from sweep
-// `sweep0` of frame index f0: every voxel in every step, the state moving between the two slot buffers.
-template <int K, int NT>
-__device__ __noinline__ void finish_dense(const ListParams& P, const Rep& R, uint32_t ci, uint32_t f0, uint32_t sweep0,
-                                          uint32_t* s_diag) {
-    const uint32_t X = R.rd.X, Y = R.rd.Y, Z = R.rd.Z, V = X * Y * Z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t k0 = R.rd.seed_lo, k1 = R.rd.seed_hi;
-    uint8_t* cur = P.lat + R.rd.base * K;
-    uint8_t* nx = P.lat2 + R.rd.base * K;
-    auto decide = [&](const Vox<K>& c, uint32_t x, uint32_t y, uint32_t z, uint32_t v, uint32_t fr, uint32_t sweep) -> uint32_t {
-        if (vox_empty<K>(c)) return 0u;
-        return moves_along<K>(R, c, x, y, z, v, fr, sweep, sweep_word(d_philox(v, fr, 0u, 0u, k0, k1), sweep));
-    };
-    for (uint32_t f = f0; f < P.n_frames; f++) {
-        const uint32_t fr = P.frame0 + f;
-        for (uint32_t sweep = f == f0 ? sweep0 : 0u; sweep < 3u; sweep++) {
-            const uint32_t dx = sweep == 0u, dy = sweep == 1u, dz = sweep == 2u;
-            const uint32_t stride = sweep == 0u ? Y * Z : sweep == 1u ? Z : 1u;
-            __syncthreads();
-            for (uint32_t v = tid; v < V; v += NT) {
-                const uint32_t xy = v / Z, z = v - xy * Z, x = xy / Y, y = xy - x * Y;
-                const bool has_lo = (dx ? x : dy ? y : z) > 0u, has_hi = dx ? x + 1u < X : dy ? y + 1u < Y : z + 1u < Z;
-                const Vox<K> own = ls_load<K>(cur + (uint64_t)v * K);
-                const Vox<K> lo = has_lo ? ls_load<K>(cur + (uint64_t)(v - stride) * K) : vox_zero<K>();
-                const Vox<K> hi = has_hi ? ls_load<K>(cur + (uint64_t)(v + stride) * K) : vox_zero<K>();
-                const uint32_t dme = decide(own, x, y, z, v, fr, sweep);
-                const uint32_t dlo = has_lo ? decide(lo, x - dx, y - dy, z - dz, v - stride, fr, sweep) : 0u;
-                const uint32_t dhi = has_hi ? decide(hi, x + dx, y + dy, z + dz, v + stride, fr, sweep) : 0u;
-                st_vox_g<K>(nx + (uint64_t)v * K, combine<K>(own, dme, lo, dlo, hi, dhi, v, v - stride, v + stride, fr, sweep));
-            }
-            __syncthreads();
-            uint8_t* const t = cur;
-            cur = nx;
-            nx = t;
-        }
-        for (uint32_t base = warp * 32u; base < V; base += NT) {
-            const uint32_t v = base + lane;
-            Vox<K> c = vox_zero<K>();
-            uint32_t w3 = 0u;
-            bool react = false;
-            if (v < V) {
-                c = ls_load<K>(cur + (uint64_t)v * K);
-                if (!vox_empty<K>(c)) {
-                    w3 = d_philox(v, fr, 0u, 0u, k0, k1).w;
-                    react = !list_calm<K>(P.T, ci, c, w3);
-                }
-            }
-            for (uint32_t m = __ballot_sync(0xffffffffu, react); m; m &= m - 1u) {
-                const uint32_t u = base + (uint32_t)__ffs((int)m) - 1u;
-                Vox<K> r = ls_load<K>(cur + (uint64_t)u * K);
-                const uint32_t uw3 = __shfl_sync(0xffffffffu, w3, (int)(u - base));
-                const bool fired = react_voxel_warp<K>(r, 0u, u, fr, k0, k1, R.rd.rate_mult, P.T, nullptr,
-                                                       P.counts + (size_t)ci * R.S1, s_diag, uw3);
-                __syncwarp();
-                if (lane == 0u && fired) st_vox_g<K>(cur + (uint64_t)u * K, r);
-                __syncwarp();
-            }
-        }
-    }
-    __syncthreads();
-    if (cur != P.lat + R.rd.base * K)
-        for (uint32_t v = tid; v < V; v += NT)
-            st_vox_g<K>(P.lat + (R.rd.base + v) * K, ls_load<K>(cur + (uint64_t)v * K));
-}
-
 template <int K, int NT>
 __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) list_frames_kernel(const __grid_constant__ ListParams P) {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -220,16 +155,7 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) list_frames_kernel(const
         return 0u;
     };
     auto voxel = [&](uint32_t t) -> uint32_t { return ((t >> 20) * Y + ((t >> 10) & 1023u)) * Z + (t & 1023u); };
-    auto finish = [&]() {
-        __syncthreads();
-        if (tid < PD_N && s_diag[tid]) atomicAdd(P.diag + tid, s_diag[tid]);
-    };
-    if (n_in == LIST_DENSE) {
-        __syncthreads();
-        finish_dense<K, NT>(P, R, ci, 0u, 0u, s_diag);
-        finish();
-        return;
-    }
+    if (n_in & LIST_STOPPED) return;
     clear_hash();
     __syncthreads();
     uint32_t np = 0u;
@@ -261,9 +187,8 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) list_frames_kernel(const
         return w;
     };
     uint32_t n = n_in;  // entries; the same value in every thread
-    // The occupied entries to the front of the list, the hash made anew.  Returns false when they and as
-    // many new entries as there are particles do not fit.
-    auto compact = [&](uint32_t fr) -> bool {
+    // The occupied entries to the front of the list, the hash made anew.
+    auto compact = [&](uint32_t fr) {
         for (uint32_t i = tid; i < n; i += NT)
             if (tch[i]) c[i] = nc[i];
         if (tid == 0u) cnt[1] = 0u;
@@ -291,24 +216,18 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) list_frames_kernel(const
         }
         if (tid == 0u) cnt[0] = n;
         __syncthreads();
-        return n + cnt[4] <= cap;
     };
 
     const uint32_t* const rowu = R.thr + (R.code * R.NC + R.code) * R.S1;
-    uint32_t over_f = 0u, over_sweep = 0u;
-    bool over = false;
-    for (uint32_t f = 0; f < P.n_frames && !over; f++) {
+    uint32_t f = 0;
+    for (; f < P.n_frames; f++) {
         const uint32_t fr = P.frame0 + f;
+        if (2u * cnt[4] > cap) break;  // the frame might not fit; particles are the same in all its sweeps
         for (uint32_t sweep = 0; sweep < 3u; sweep++) {
             // an axis of length 1 has no neighbour: every decision is 0 and every content stays
             if ((sweep == 0u ? R.rd.X : sweep == 1u ? Y : Z) == 1u) continue;
             // a sweep makes at most one entry per particle
-            if (n + cnt[4] > cap && !compact(fr)) {
-                over = true;
-                over_f = f;
-                over_sweep = sweep;
-                break;
-            }
+            if (n + cnt[4] > cap) compact(fr);
             const uint32_t stride = sweep == 0u ? Y * Z : sweep == 1u ? Z : 1u;
             const uint32_t shift = sweep == 0u ? 20u : sweep == 1u ? 10u : 0u;
             const uint32_t dim = sweep == 0u ? R.rd.X : sweep == 1u ? Y : Z;
@@ -388,7 +307,6 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) list_frames_kernel(const
             }
             __syncthreads();
         }
-        if (over) break;
         // reactions
         uint32_t* const n_pend = &cnt[2u + (f & 1u)];
         if (tid == 0u) cnt[2u + ((f & 1u) ^ 1u)] = 0u;
@@ -423,21 +341,6 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) list_frames_kernel(const
         // emptied entries out while no Philox block is lost; the sweeps make sure of the room
         if (f + 1u < P.n_frames && 2u * n > 3u * cnt[4]) compact(fr);
     }
-    if (over) {
-        // the particles have outgrown the block: its lattice, then the rest of the call over the lattice
-        const uint32_t V = R.rd.X * Y * Z;
-        for (uint32_t v = tid; v < V; v += NT) st_vox_g<K>(P.lat + (R.rd.base + v) * K, vox_zero<K>());
-        __syncthreads();
-        for (uint32_t i = tid; i < n; i += NT) st_vox_g<K>(P.lat + (R.rd.base + voxel(xyz[i])) * K, c[i]);
-        __syncthreads();
-        finish_dense<K, NT>(P, R, ci, over_f, over_sweep, s_diag);
-        if (tid == 0u) {
-            P.n[rep] = LIST_DENSE;
-            *P.host_flag = 1u;
-        }
-        finish();
-        return;
-    }
     __syncthreads();
     if (tid == 0u) cnt[1] = 0u;
     __syncthreads();
@@ -449,8 +352,15 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) list_frames_kernel(const
         st_vox_g<K>(P.cont + (gl + p) * K, w);
     }
     __syncthreads();
-    if (tid == 0u) P.n[rep] = cnt[1];
-    finish();
+    if (tid == 0u) {
+        const bool stopped = f < P.n_frames;
+        P.n[rep] = stopped ? cnt[1] | LIST_STOPPED : cnt[1];
+        if (stopped) {
+            P.at[rep] = P.frame0 + f;
+            *P.host_flag = 1u;
+        }
+    }
+    if (tid < PD_N && s_diag[tid]) atomicAdd(P.diag + tid, s_diag[tid]);
 }
 
 // Appends the occupied voxels of every replicate's slots to its list (blockIdx.y: replicates).
@@ -486,6 +396,7 @@ __global__ void list_check_kernel(const ListParams P, uint32_t n_rep) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < n_rep && P.n[r] > P.cap) {
         P.n[r] = LIST_DENSE;
+        P.at[r] = P.frame0;
         *P.host_flag = 1u;
     }
 }
@@ -506,8 +417,8 @@ __global__ void __launch_bounds__(256) list_zero_kernel(const ListParams P, uint
 template <int K>
 __global__ void __launch_bounds__(256) list_unpack_kernel(const ListParams P, uint32_t n_rep) {
     for (uint32_t rep = blockIdx.y; rep < n_rep; rep += gridDim.y) {
-        const uint32_t n = P.n[rep];
-        if (n == LIST_DENSE) continue;
+        if (P.n[rep] == LIST_DENSE) continue;
+        const uint32_t n = P.n[rep] & ~LIST_STOPPED;
         const RepDesc rd = P.reps[rep];
         const uint64_t gl = (uint64_t)rep * P.cap;
         for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u) {
@@ -518,17 +429,11 @@ __global__ void __launch_bounds__(256) list_unpack_kernel(const ListParams P, ui
     }
 }
 
-// View 0 (views.cuh) of replicate 0 into zeroed floats, from its list or, LIST_DENSE, from its slots.
+// View 0 (views.cuh) of replicate 0 into zeroed floats, from its list.
 template <int K>
 __global__ void __launch_bounds__(256) list_view_kernel(const ListParams P, float* out) {
     const RepDesc rd = P.reps[0];
-    const uint32_t n = P.n[0];
-    if (n == LIST_DENSE) {
-        const uint32_t V = rd.X * rd.Y * rd.Z;
-        for (uint32_t v = blockIdx.x * 256u + threadIdx.x; v < V; v += gridDim.x * 256u)
-            out[v] = __fdiv_rn((float)view_majority<K>(ls_load<K>(P.lat + (rd.base + v) * K).w), 255.0f);
-        return;
-    }
+    const uint32_t n = P.n[0] == LIST_DENSE ? 0u : P.n[0] & ~LIST_STOPPED;
     for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u) {
         const uint32_t t = P.xyz[i];
         out[((t >> 20) * rd.Y + ((t >> 10) & 1023u)) * rd.Z + (t & 1023u)] =

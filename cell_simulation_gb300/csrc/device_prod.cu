@@ -231,15 +231,17 @@ struct DeviceProd {
     DevBuf<uint32_t> mul, react, resv_bits;
     cudaGraphExec_t ip_graph[8] = {};  // of 1 .. kInplaceGraphFrames frames
     int ip_graph_cur[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
-    // the list form: voxels, contents and lengths of every replicate's list (l_cap entries each), a
-    // host-visible word that it sets when a replicate outgrew its list; ls_state: the lattice is in the
-    // lists.  p_max: the most particles of a replicate, as last seen by the host.
-    DevBuf<uint32_t> l_xyz, l_n;
+    // the list form: voxels, contents and lengths of every replicate's list (l_cap entries each), the frames
+    // that stopped replicates stand at, and a host-visible word that is set when one has stopped; ls_state: the
+    // lattice is in the lists.  p_max: the most particles of a replicate, as last seen by the host.
+    DevBuf<uint32_t> l_xyz, l_n, l_at;
     DevBuf<uint8_t> l_cont;
     uint32_t l_cap = 0;
     uint32_t* h_flag = nullptr;
     bool ls_state = false;
     uint64_t p_max = 0;
+    cudaEvent_t piece_ev[2] = {};  // ends of the last two launches of a long call
+    DevBuf<uint32_t> ip_from;      // InplaceParams::from while replicates are brought to one frame, else empty
     DevBuf<uint32_t> exchange;  // workspace of lattice uploads and read-backs (see exchange_piece)
     uint32_t one_code = 0;  // the region code of every voxel of a single lattice when they share one, else 0
     DevBuf<uint8_t> spec;  // species of the voxels of one particle, 32 bytes per bitmap word
@@ -281,6 +283,8 @@ struct DeviceProd {
         if (h_flag) cudaFreeHost(h_flag);
         if (h_frames) cudaFreeHost(h_frames);
         for (cudaEvent_t e : frame_ev)
+            if (e) cudaEventDestroy(e);
+        for (cudaEvent_t e : piece_ev)
             if (e) cudaEventDestroy(e);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -609,6 +613,8 @@ static void build_groups(DeviceProd* d);
 static void build_units(DeviceProd* d);
 static void build_lists(DeviceProd* d);
 static void ensure_slots(DeviceProd* d);
+static bool lists_settle(DeviceProd* d);
+static void settle(DeviceProd* d);
 
 // The fused Y and Z sweeps need every group to hold whole rows.
 static bool fused_fits(const DeviceProd* d) {
@@ -920,6 +926,7 @@ static void build_lists(DeviceProd* d) {
     if (d->l_xyz.n < n) d->l_xyz.alloc(n);
     if (d->l_cont.n < n * d->K) d->l_cont.alloc(n * d->K);
     if (d->l_n.n < d->n_rep) d->l_n.alloc(d->n_rep);
+    if (d->l_at.n < d->n_rep) d->l_at.alloc(d->n_rep);
     if (!d->h_flag) CS_CUDA(cudaHostAlloc(&d->h_flag, 4, cudaHostAllocMapped));
     *d->h_flag = 0u;
     d->n_items = d->n_rep;
@@ -1492,6 +1499,7 @@ void prod_set_lattice(DeviceProd* d, const Model& m, const uint32_t* slots) {
     DeviceGuard g(d->device);
     const uint64_t V = m.V, piece = exchange_piece(V, m.K);
     if (d->exchange.n < piece * m.K) d->exchange.alloc(piece * m.K);
+    settle(d);  // the frames enqueued before count in the diagnostics
     CS_CUDA(cudaStreamSynchronize(d->stream));
     d->cur = 0;
     d->frame_known = false;
@@ -1520,8 +1528,16 @@ void prod_set_lattice(DeviceProd* d, const Model& m, const uint32_t* slots) {
     for (uint32_t s = 1; s < d->S1; s++) d->p_max += c[s];
 }
 
+static void get_lattice_once(DeviceProd* d, const Model& m, uint32_t* slots, uint32_t* occ, int32_t* conc);
+
 void prod_get_lattice(DeviceProd* d, const Model& m, uint32_t* slots, uint32_t* occ, int32_t* conc) {
     DeviceGuard g(d->device);
+    do {
+        get_lattice_once(d, m, slots, occ, conc);
+    } while (lists_settle(d));
+}
+
+static void get_lattice_once(DeviceProd* d, const Model& m, uint32_t* slots, uint32_t* occ, int32_t* conc) {
     ensure_slots(d);
     const uint64_t V = m.V, words = (uint64_t)m.K + 1u + d->S1, piece = exchange_piece(V, words);
     if (d->exchange.n < piece * words) d->exchange.alloc(piece * words);
@@ -1548,6 +1564,7 @@ void prod_get_lattice(DeviceProd* d, const Model& m, uint32_t* slots, uint32_t* 
 
 void prod_seed(DeviceProd* d, uint64_t seed) {
     if (d->seed_set && seed == d->cur_seed) return;
+    settle(d);
     for (auto& r : d->h_reps) {
         r.seed_lo = (uint32_t)seed;
         r.seed_hi = (uint32_t)(seed >> 32);
@@ -1562,15 +1579,23 @@ void prod_seed(DeviceProd* d, uint64_t seed) {
 
 // Runs n frames; batched = one launch per frame over all replicates (a
 // captured two-frame graph replays pairs), otherwise one launch per replicate.
-static void run_frames_nosync(DeviceProd* d, uint32_t n, bool batched);
+static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold = false);
 
-static void run_frames(DeviceProd* d, uint32_t n, uint64_t frame0, bool batched) {
-    if (n == 0) return;
+// The next frame is frame0: its number into stepbuf[cur] unless it is there.  Waits for the stream.
+static void start_at(DeviceProd* d, uint64_t frame0) {
+    settle(d);
+    if (!d->ls_state) CS_CUDA(cudaStreamSynchronize(d->stream));
+    if (d->frame_known && d->next_frame == frame0) return;
     uint32_t f32 = (uint32_t)frame0;
     CS_CUDA(cudaMemcpyAsync(d->stepbuf.p + d->cur, &f32, 4, cudaMemcpyHostToDevice, d->stream));
     CS_CUDA(cudaStreamSynchronize(d->stream));
     d->next_frame = frame0;
     d->frame_known = true;
+}
+
+static void run_frames(DeviceProd* d, uint32_t n, uint64_t frame0, bool batched) {
+    if (n == 0) return;
+    start_at(d, frame0);
     run_frames_nosync(d, n, batched);
 }
 
@@ -1626,6 +1651,7 @@ static InplaceParams inplace_params(const DeviceProd* d) {
     P.fa = d->stepbuf.p + d->cur;
     P.fb = d->stepbuf.p + (d->cur ^ 1);
     P.thr_smem = thr_words(d) != 0u;
+    P.from = d->ip_from.n ? d->ip_from.p : nullptr;
     return P;
 }
 
@@ -1634,12 +1660,12 @@ static ListParams lists_params(const DeviceProd* d) {
     P.T = d->T;
     P.reps = d->reps.p;
     P.lat = d->slots[d->cur].p;
-    P.lat2 = d->slots[d->cur ^ 1].p;
     P.region_pad = d->region_pad.p;
     P.code = d->one_code;
     P.xyz = d->l_xyz.p;
     P.cont = d->l_cont.p;
     P.n = d->l_n.p;
+    P.at = d->l_at.p;
     P.cap = d->l_cap;
     P.counts = d->counts.p;
     P.diag = d->diag.p;
@@ -1728,34 +1754,36 @@ static void run_inplace(DeviceProd* d, uint32_t n, bool batched) {
     d->ip_epoch = d->seed_epoch;
 }
 
-// n frames of the list form; false when the particles have outgrown it (nothing is enqueued then).
+// n frames (at most LIST_MAX_FRAMES) of the list form; false, with nothing enqueued, when a replicate has
+// stopped or the particles need longer lists than fit.
 static bool run_lists(DeviceProd* d, uint32_t n, bool batched) {
-    if (*static_cast<volatile uint32_t*>(d->h_flag)) return false;
+    const volatile uint32_t* const stopped = d->h_flag;
+    if (*stopped) return false;
     if (d->p_max * 9u > 4ull * d->l_cap) {  // less than 2.25 entries per particle: larger lists, or none
-        const uint32_t cap = lists_cap(d);
-        if (cap <= d->l_cap) return false;
+        if (lists_cap(d) <= d->l_cap) return false;
+        CS_CUDA(cudaStreamSynchronize(d->stream));
+        if (*stopped) return false;
         build_lists(d);
     }
     if (!d->ls_state) {
         ensure_slots(d);
-        lists_pack((int)d->K, lists_params(d), d->n_rep, max_rep_voxels(d), d->stream);
+        ListParams P = lists_params(d);
+        P.frame0 = (uint32_t)d->next_frame;
+        lists_pack((int)d->K, P, d->n_rep, max_rep_voxels(d), d->stream);
     }
     ListParams P = lists_params(d);
+    P.frame0 = (uint32_t)d->next_frame;
+    P.n_frames = n;
     // more threads where SMs have at most one block anyway: fewer rounds of a sweep's entries and more warps
     // for the SSAs, against dearer barriers (us per frame with 512 / 768 threads, 96 replicates of the 12-species
     // network on 12 .. 24 cubed voxels: 300 particles 11.5 / 11.9, 450 15.7 / 14.0, 600 20.0 / 19.1, 780 25.1 / 22.9)
     const int threads = d->n_rep > (uint32_t)d->num_sms || d->p_max <= 128 ? 256 : d->p_max <= 350 ? 512 : 768;
-    for (uint32_t k = 0; k < n; k += P.n_frames) {
-        P.frame0 = (uint32_t)(d->next_frame + k);
-        P.n_frames = std::min(n - k, LIST_MAX_FRAMES);
-        if (batched) {
-            P.rep0 = 0;
-            lists_launch((int)d->K, threads, P, d->n_rep, d->stream);
-        } else {
-            for (uint32_t r = 0; r < d->n_rep; r++) {
-                P.rep0 = r;
-                lists_launch((int)d->K, threads, P, 1, d->stream);
-            }
+    if (batched) {
+        lists_launch((int)d->K, threads, P, d->n_rep, d->stream);
+    } else {
+        for (uint32_t r = 0; r < d->n_rep; r++) {
+            P.rep0 = r;
+            lists_launch((int)d->K, threads, P, 1, d->stream);
         }
     }
     d->next_frame += n;
@@ -1767,18 +1795,43 @@ static bool run_lists(DeviceProd* d, uint32_t n, bool batched) {
     return true;
 }
 
+// n frames of the list form in launches of LIST_MAX_FRAMES; while one runs the host looks whether the launch
+// before has stopped, so that at most two launches are made in vain.  Returns the frames that were not
+// enqueued: the particles have outgrown the lists.
+static uint32_t run_list_pieces(DeviceProd* d, uint32_t n, bool batched) {
+    uint32_t pieces = 0;
+    while (n) {
+        const uint32_t m = std::min(n, LIST_MAX_FRAMES);
+        if (!run_lists(d, m, batched)) return n;
+        n -= m;
+        if (n == 0) break;
+        cudaEvent_t& ev = d->piece_ev[pieces & 1u];
+        if (!ev) CS_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        CS_CUDA(cudaEventRecord(ev, d->stream));
+        if (pieces) CS_CUDA(cudaEventSynchronize(d->piece_ev[(pieces & 1u) ^ 1u]));
+        pieces++;
+    }
+    return 0;
+}
+
+static bool lists_stopped(const DeviceProd* d) { return d->ls_state && *static_cast<volatile uint32_t*>(d->h_flag) != 0u; }
+
 // Enqueues n frames; the frame number must already be in stepbuf[cur] (and
-// its host copy in next_frame).
-static void run_frames_nosync(DeviceProd* d, uint32_t n, bool batched) {
-    if (n == 0) return;
-    if (all_cfgs()[d->cfg_index].kind == KIND_LISTS) {
-        if (run_lists(d, n, batched)) return;
+// its host copy in next_frame).  Where lists have stopped, the frames that they
+// lack come first; with hold they do not, nothing more is enqueued, and the
+// stream is idle: returns whether that is so.
+static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold) {
+    if (n == 0) return false;
+    while (all_cfgs()[d->cfg_index].kind == KIND_LISTS) {
+        n = run_list_pieces(d, n, batched);
+        if (n == 0) return false;
         CS_CUDA(cudaStreamSynchronize(d->stream));
-        set_cfg(d, pick_default_cfg(d, false));
+        if (hold && lists_stopped(d)) return true;
+        if (!lists_settle(d)) set_cfg(d, pick_default_cfg(d, false));
     }
     if (all_cfgs()[d->cfg_index].kind == KIND_INPLACE) {
         run_inplace(d, n, batched);
-        return;
+        return false;
     }
     ensure_slots(d);
     d->ip_state = d->ip_valid = d->ls_state = false;
@@ -1788,7 +1841,7 @@ static void run_frames_nosync(DeviceProd* d, uint32_t n, bool batched) {
         d->next_frame += n;
         d->occ_valid = false;  // the resident form keeps no occupancy bitmaps and no x-decisions
         d->xdec_valid = false;
-        return;
+        return false;
     }
     // the brick pass and the sweep stream read and maintain the occupancy bitmaps
     const int kind = all_cfgs()[d->cfg_index].kind;
@@ -1868,6 +1921,7 @@ static void run_frames_nosync(DeviceProd* d, uint32_t n, bool batched) {
         d->xdec_frame = d->next_frame;
         d->xdec_epoch = d->seed_epoch;
     }
+    return false;
 }
 
 // The frame number of the next frame into stepbuf[cur] (the step's one
@@ -1889,15 +1943,103 @@ static void upload_frame(DeviceProd* d, uint64_t frame0) {
     d->frame_known = true;
 }
 
+// The counts of every replicate and the wait-timeout word behind them into h_counts, and p_max from them.
+static void fetch_counts(DeviceProd* d) {
+    const size_t n = (size_t)d->n_rep * d->S1;
+    if (!d->h_counts) CS_CUDA(cudaMallocHost(&d->h_counts, (n + 1) * 8));
+    CS_CUDA(cudaMemcpyAsync(d->h_counts, d->counts.p, (n + 1) * 8, cudaMemcpyDeviceToHost, d->stream));
+    CS_CUDA(cudaStreamSynchronize(d->stream));
+    d->p_max = 0;
+    for (size_t r = 0; r < d->n_rep; r++) {
+        uint64_t p = 0;
+        for (uint32_t s = 1; s < d->S1; s++) p += d->h_counts[r * d->S1 + s];
+        d->p_max = std::max(d->p_max, p);
+    }
+}
+
+// After a stop, with the stream idle: the handle goes back to the earliest frame at which a replicate stands
+// (next_frame) and, with one replicate, to the form that its particles now call for: longer lists, or none.
+// Several replicates stand at frames of their own: their first frames are left in ip_from and the handle takes
+// the in-place form.
+static void lists_leave(DeviceProd* d) {
+    std::vector<uint32_t> n(d->n_rep), at(d->n_rep);
+    CS_CUDA(cudaMemcpyAsync(n.data(), d->l_n.p, d->n_rep * 4, cudaMemcpyDeviceToHost, d->stream));
+    CS_CUDA(cudaMemcpyAsync(at.data(), d->l_at.p, d->n_rep * 4, cudaMemcpyDeviceToHost, d->stream));
+    fetch_counts(d);
+    const uint32_t next = (uint32_t)d->next_frame;
+    uint32_t lag = 0;
+    for (uint32_t r = 0; r < d->n_rep; r++) {
+        if (!(n[r] & LIST_STOPPED)) at[r] = next;
+        lag = std::max(lag, next - at[r]);
+    }
+    d->slots_stale = true;  // a reader may have had the slots written, from the same lists
+    if (d->n_rep == 1u) {
+        const bool longer = lists_cap(d) > d->l_cap;
+        ensure_slots(d);
+        d->ls_state = false;
+        set_cfg(d, pick_default_cfg(d, longer));
+    } else {
+        ensure_slots(d);
+        d->ls_state = false;
+        set_cfg(d, find_cfg(d->K, KIND_INPLACE, 0));
+        d->ip_from.alloc(d->n_rep);
+        CS_CUDA(cudaMemcpyAsync(d->ip_from.p, at.data(), d->n_rep * 4, cudaMemcpyHostToDevice, d->stream));
+        CS_CUDA(cudaStreamSynchronize(d->stream));
+    }
+    *d->h_flag = 0u;
+    d->frame_known = false;
+    upload_frame(d, d->next_frame - lag);
+}
+
+// With the stream idle: runs the frames that stopped replicates lack, so that every replicate stands at
+// next_frame (the stream is idle again); false when there is none.  One replicate runs them in pieces, each in
+// the form that its growing population calls for by then (an idle GPU per piece costs 2% at 20 us per frame).
+// Several are brought to one frame by the in-place form, which each joins at its own.
+static constexpr uint32_t kSettlePiece = 32;
+static bool lists_settle(DeviceProd* d) {
+    if (!lists_stopped(d)) return false;
+    const uint64_t next = d->next_frame;
+    const uint32_t cap = d->l_cap;
+    lists_leave(d);
+    if (d->n_rep == 1u) {
+        while (d->next_frame < next) {
+            run_frames_nosync(d, (uint32_t)std::min<uint64_t>(next - d->next_frame, kSettlePiece), true, true);
+            CS_CUDA(cudaStreamSynchronize(d->stream));
+            if (lists_stopped(d)) {
+                lists_leave(d);
+                continue;
+            }
+            fetch_counts(d);
+            const int idx = pick_default_cfg(d, true);
+            if (idx != d->cfg_index) set_cfg(d, idx);
+        }
+        return true;
+    }
+    run_inplace(d, (uint32_t)(next - d->next_frame), true);
+    CS_CUDA(cudaStreamSynchronize(d->stream));
+    d->ip_from.reset();
+    drop_graphs(d);
+    fetch_counts(d);
+    const int idx = pick_default_cfg(d, lists_cap(d) > cap);
+    if (idx != d->cfg_index) set_cfg(d, idx);
+    return true;
+}
+
+// Before anything that reads or changes the state, its seed or its frame number in another way than the list
+// form's own launches do.  Waits for the stream where the lattice is in lists.
+static void settle(DeviceProd* d) {
+    if (!d->ls_state) return;
+    do CS_CUDA(cudaStreamSynchronize(d->stream));
+    while (lists_settle(d));
+}
+
 void prod_step(DeviceProd* d, uint32_t n_steps, uint64_t seed, int precision, uint64_t frame0, uint32_t write_freq,
                const std::vector<uint32_t>& logging, std::vector<cs_stat_sample>& samples) {
     DeviceGuard g(d->device);
     if (n_steps == 0) return;
     prod_seed(d, seed);
-    if (d->T.precision != precision) {
-        d->T.precision = precision;
-        drop_graphs(d);
-    }
+    prod_set_precision(d, precision);
+    if (d->next_frame != frame0) settle(d);
     std::vector<uint64_t> sample_frames;
     if (write_freq)
         for (uint64_t f = frame0; f < frame0 + n_steps; f++)
@@ -1908,21 +2050,32 @@ void prod_step(DeviceProd* d, uint32_t n_steps, uint64_t seed, int precision, ui
     upload_frame(d, frame0);
     if (!sample_frames.empty() && d->sample_ring.n < sample_frames.size() * d->S1)
         d->sample_ring.alloc(sample_frames.size() * d->S1);
-    for (size_t i = 0; i < sample_frames.size(); i++) {
-        run_frames_nosync(d, (uint32_t)(sample_frames[i] - f), true);
-        f = sample_frames[i];
-        CS_CUDA(cudaMemcpyAsync(d->sample_ring.p + i * d->S1, d->counts.p, d->S1 * 8, cudaMemcpyDeviceToDevice,
-                                d->stream));
+    if (sample_frames.empty()) {
+        run_frames_nosync(d, n_steps, true);
+        return;
     }
-    run_frames_nosync(d, (uint32_t)(end - f), true);
-    if (!sample_frames.empty()) {
-        std::vector<unsigned long long> h(sample_frames.size() * d->S1);
-        CS_CUDA(cudaMemcpyAsync(h.data(), d->sample_ring.p, h.size() * 8, cudaMemcpyDeviceToHost, d->stream));
+    std::vector<unsigned long long> h(sample_frames.size() * d->S1);
+    for (size_t i = 0;;) {
+        bool held = false;
+        for (; i <= sample_frames.size(); i++) {
+            const bool last = i == sample_frames.size();
+            const uint64_t to = last ? end : sample_frames[i];
+            held = run_frames_nosync(d, (uint32_t)(to - f), true, true);
+            if (held) break;
+            f = to;
+            if (last) CS_CUDA(cudaMemcpyAsync(h.data(), d->sample_ring.p, h.size() * 8, cudaMemcpyDeviceToHost, d->stream));
+            else CS_CUDA(cudaMemcpyAsync(d->sample_ring.p + i * d->S1, d->counts.p, d->S1 * 8, cudaMemcpyDeviceToDevice, d->stream));
+        }
         CS_CUDA(cudaStreamSynchronize(d->stream));
-        for (size_t i = 0; i < sample_frames.size(); i++)
-            for (uint32_t sp : logging)
-                samples.push_back(cs_stat_sample{sp, (int32_t)(long long)h[i * d->S1 + sp], (uint32_t)sample_frames[i]});
+        if (!lists_stopped(d)) break;
+        // the lists stopped before some of the samples: on from that frame (a sample shows the counts before its own)
+        lists_leave(d);
+        f = d->next_frame;
+        i = (size_t)(std::upper_bound(sample_frames.begin(), sample_frames.end(), f) - sample_frames.begin());
     }
+    for (size_t i = 0; i < sample_frames.size(); i++)
+        for (uint32_t sp : logging)
+            samples.push_back(cs_stat_sample{sp, (int32_t)(long long)h[i * d->S1 + sp], (uint32_t)sample_frames[i]});
 }
 
 static const char* const kWaitFault =
@@ -1930,25 +2083,18 @@ static const char* const kWaitFault =
 
 void prod_get_counts(DeviceProd* d, int64_t* counts) {
     DeviceGuard g(d->device);
+    do fetch_counts(d);
+    while (lists_settle(d));
     const size_t n = (size_t)d->n_rep * d->S1;
-    if (!d->h_counts) CS_CUDA(cudaMallocHost(&d->h_counts, (n + 1) * 8));
-    // the counts and the wait-timeout word in one copy
-    CS_CUDA(cudaMemcpyAsync(d->h_counts, d->counts.p, (n + 1) * 8, cudaMemcpyDeviceToHost, d->stream));
-    CS_CUDA(cudaStreamSynchronize(d->stream));
     if (d->h_counts[n]) throw Error(CS_ERR_CUDA, kWaitFault);
     for (size_t i = 0; i < n; i++) counts[i] = (int64_t)d->h_counts[i];
-    d->p_max = 0;
-    for (size_t r = 0; r < d->n_rep; r++) {
-        uint64_t p = 0;
-        for (uint32_t s = 1; s < d->S1; s++) p += d->h_counts[r * d->S1 + s];
-        d->p_max = std::max(d->p_max, p);
-    }
 }
 
 void prod_set_counts(DeviceProd* d, const int64_t* counts) {
     DeviceGuard g(d->device);
     std::vector<unsigned long long> h((size_t)d->n_rep * d->S1);
     for (size_t i = 0; i < h.size(); i++) h[i] = (unsigned long long)counts[i];
+    settle(d);
     CS_CUDA(cudaStreamSynchronize(d->stream));
     CS_CUDA(cudaMemcpy(d->counts.p, h.data(), h.size() * 8, cudaMemcpyHostToDevice));
 }
@@ -1970,6 +2116,7 @@ void prod_render_view(DeviceProd* d, int32_t view, int32_t slice_axis, uint32_t 
         else inplace_view((int)d->K, inplace_params(d), r, out_dev, d->stream);
         if (!out_device) CS_CUDA(cudaMemcpyAsync(out_host, out_dev, V * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
         CS_CUDA(cudaStreamSynchronize(d->stream));
+        if (lists_settle(d)) prod_render_view(d, view, slice_axis, slice, out_host, out_device);
         return;
     }
     ensure_slots(d);
@@ -1989,21 +2136,26 @@ void prod_render_view(DeviceProd* d, int32_t view, int32_t slice_axis, uint32_t 
     CS_LAUNCH_CHECK();
     if (!out_device) CS_CUDA(cudaMemcpyAsync(out_host, out_dev, V * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
     CS_CUDA(cudaStreamSynchronize(d->stream));
+    if (lists_settle(d)) prod_render_view(d, view, slice_axis, slice, out_host, out_device);
 }
 
 void prod_get_diag(DeviceProd* d, uint32_t* diag, uint32_t n) {
     DeviceGuard g(d->device);
     uint32_t h[PD_N];
-    CS_CUDA(cudaMemcpyAsync(h, d->diag.p, sizeof(h), cudaMemcpyDeviceToHost, d->stream));
-    CS_CUDA(cudaStreamSynchronize(d->stream));
+    do {
+        CS_CUDA(cudaMemcpyAsync(h, d->diag.p, sizeof(h), cudaMemcpyDeviceToHost, d->stream));
+        CS_CUDA(cudaStreamSynchronize(d->stream));
+    } while (lists_settle(d));
     for (uint32_t i = 0; i < n; i++) diag[i] = i < PD_N ? h[i] : 0u;
 }
 
 void prod_sync(DeviceProd* d) {
     DeviceGuard g(d->device);
     unsigned long long fault = 0;
-    CS_CUDA(cudaMemcpyAsync(&fault, d->counts.p + (size_t)d->n_rep * d->S1, 8, cudaMemcpyDeviceToHost, d->stream));
-    CS_CUDA(cudaStreamSynchronize(d->stream));
+    do {
+        CS_CUDA(cudaMemcpyAsync(&fault, d->counts.p + (size_t)d->n_rep * d->S1, 8, cudaMemcpyDeviceToHost, d->stream));
+        CS_CUDA(cudaStreamSynchronize(d->stream));
+    } while (lists_settle(d));
     if (fault) throw Error(CS_ERR_CUDA, kWaitFault);
 }
 
@@ -2082,10 +2234,11 @@ void prod_ensemble_step(DeviceProd* d, uint32_t n_steps, bool batched, uint64_t 
 }
 
 void prod_set_precision(DeviceProd* d, int precision) {
-    if (d->T.precision != precision) {
-        d->T.precision = precision;
-        drop_graphs(d);
-    }
+    if (d->T.precision == precision) return;
+    DeviceGuard g(d->device);
+    settle(d);
+    d->T.precision = precision;
+    drop_graphs(d);
 }
 
 uint64_t prod_total_voxels(const DeviceProd* d) { return d->total_voxels; }
@@ -2096,8 +2249,10 @@ uint32_t prod_s1(const DeviceProd* d) { return d->S1; }
 // Downloads the packed slots of every replicate (K bytes per voxel).
 void prod_get_slots_raw(DeviceProd* d, uint8_t* out) {
     DeviceGuard g(d->device);
-    ensure_slots(d);
-    CS_CUDA(cudaStreamSynchronize(d->stream));
+    do {
+        ensure_slots(d);
+        CS_CUDA(cudaStreamSynchronize(d->stream));
+    } while (lists_settle(d));
     CS_CUDA(cudaMemcpy(out, d->slots[d->cur].p, d->total_voxels * d->K, cudaMemcpyDeviceToHost));
 }
 
@@ -2108,6 +2263,7 @@ void prod_set_tiling(DeviceProd* d, int cfg_index, uint32_t seg_len) {
     const auto& c = all_cfgs();
     if (cfg_index < 0 || cfg_index >= (int)c.size() || c[cfg_index].K != (int)d->K)
         throw Error(CS_ERR_INVALID_ARG, "tile configuration does not exist for this K");
+    settle(d);
     CS_CUDA(cudaStreamSynchronize(d->stream));
     const uint32_t keep = d->seg_len;
     d->seg_len = seg_len;
@@ -2157,16 +2313,13 @@ float prod_time_frames(DeviceProd* d, uint32_t n, uint64_t frame0, bool batched)
     CS_CUDA(cudaEventCreate(&b));
     float ms = 0.0f;
     try {
-        // the frame-number upload inside run_frames synchronises; record after it
-        uint32_t f32 = (uint32_t)frame0;
-        CS_CUDA(cudaMemcpyAsync(d->stepbuf.p + d->cur, &f32, 4, cudaMemcpyHostToDevice, d->stream));
-        CS_CUDA(cudaStreamSynchronize(d->stream));
-        d->next_frame = frame0;
-        d->frame_known = true;
+        start_at(d, frame0);  // waits; record after it
         CS_CUDA(cudaEventRecord(a, d->stream));
         run_frames_nosync(d, n, batched);
-        CS_CUDA(cudaEventRecord(b, d->stream));
-        CS_CUDA(cudaEventSynchronize(b));
+        do {
+            CS_CUDA(cudaEventRecord(b, d->stream));
+            CS_CUDA(cudaEventSynchronize(b));
+        } while (lists_settle(d));
         CS_CUDA(cudaEventElapsedTime(&ms, a, b));
     } catch (...) {
         cudaEventDestroy(a);
@@ -2208,6 +2361,7 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         auto it = cache.find(key);
         if (it != cache.end()) {
             if (d->cfg_index != it->second.first) {
+                settle(d);
                 CS_CUDA(cudaStreamSynchronize(d->stream));
                 d->seg_len = 0;
                 set_cfg(d, it->second.first);
@@ -2217,7 +2371,9 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         }
     }
     if (frames == 0) frames = 1;
+    settle(d);
     CS_CUDA(cudaStreamSynchronize(d->stream));
+    const uint64_t p0 = d->p_max;  // frames of a trial may refresh it
     const size_t bytes = (size_t)d->total_voxels * d->K;
     struct Kept {
         DevBuf<uint8_t> slots;
@@ -2245,6 +2401,7 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         d->occ_valid = false;
         d->ip_state = d->ip_valid = d->ls_state = d->slots_stale = false;
         d->frame_known = false;
+        d->p_max = p0;
     };
     const int cfg0 = d->cfg_index;
     const uint32_t seg0 = d->seg_len;
@@ -2292,6 +2449,7 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
                 restore();
                 if (rep == 0 || r < t) t = r;
             }
+            if (d->cfg_index != i) continue;  // the particles outgrew the lists, and other forms were timed
             if (best < 0 || t < best_t) { best = i; best_t = t; }
         }
         if (best < 0) throw Error(CS_ERR_LIMIT, "no step variant can be set up for this lattice");

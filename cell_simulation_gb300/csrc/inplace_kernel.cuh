@@ -101,6 +101,9 @@ struct InplaceParams {
     uint32_t* fa;
     uint32_t* fb;
     uint32_t explicit_frame, frame;
+    // [n_rep] the first frame of each replicate, or null: a replicate takes part in a launch of an earlier frame
+    // only with the decisions of its first (replicates that stand at different frames are brought to one)
+    const uint32_t* from;
     uint32_t thr_smem;     // the threshold table is staged in shared memory
     uint32_t decide_only;  // Z+D: only D, for frame f = *fa
 };

@@ -306,9 +306,10 @@ cs_status cs_step_philox_timed(cs_sim* sim, uint32_t n_steps, uint64_t seed, flo
  * one block per replicate keeps the list of its occupied voxels for every
  * frame of a step call (up to about 1,000 particles per replicate at K = 16
  * and 1,300 at K = 8, edges of at most 1024 voxels, no reservoirs and no
- * reactions without reactants: cs_set_tiling refuses others; a replicate that
- * outgrows it within a call is finished over its whole lattice, and the first
- * call made after that has happened on the device takes the in-place form).  A new handle takes the resident
+ * reactions without reactants: cs_set_tiling refuses others; a replicate whose
+ * particles outgrow its list stops before the frame that might not fit, and the
+ * library runs the frames it lacks in other forms when it next looks: during a
+ * call of more than 1,024 frames, at the next call, or when the state is read).  A new handle takes the resident
  * form (small lattices), the list form or the in-place form.  Every variant
  * computes the same lattice.  cs_tiling_launches: kernel launches per frame
  * once a run is under way (the sweep stream: 3, or 2 where the Y and Z sweeps
