@@ -557,6 +557,7 @@ cs_status cs_autotune(cs_sim* sim, uint32_t frames_per_trial, int32_t* chosen_in
         need(sim, "sim");
         if (!sim->prod) throw Error(CS_ERR_STATE, "autotuning applies to the production path (cs_prepare_for_gpu(CS_RNG_PHILOX))");
         float ms = 0.0f;
+        prod_set_precision(sim->prod.get(), sim->precision);
         int best = prod_autotune(sim->prod.get(), frames_per_trial, sim->frame, true, &ms);
         if (chosen_index) *chosen_index = best;
         if (ms_per_frame) *ms_per_frame = ms;

@@ -2340,11 +2340,13 @@ namespace cellsim {
 // then 1,930 us per 51 frames where a brick variant takes 1,700), and the state
 // is restored afterwards, so tuning does not advance or change the simulation (every configuration computes the same
 // frame anyway).  Choices are cached per (K, species, reactions, regions,
-// zero-order reactions or reservoirs present, lattice shapes, device) for the
-// life of the process.
+// zero-order reactions or reservoirs present, precision, binary order of the particles, lattice shapes,
+// device) for the life of the process.
 static constexpr uint32_t kSettleFrames = 64;
 int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched, float* best_ms) {
     DeviceGuard g(d->device);
+    settle(d);
+    fetch_counts(d);
     static std::mutex mu;
     static std::map<std::string, std::pair<int, float>> cache;
     cudaDeviceProp prop{};
@@ -2354,15 +2356,17 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
                       // reservoirs and zero-order reactions make the brick pass step every interior voxel
                       "," + std::to_string(d->T.n_zero_order != 0u ? 1 : 0) + std::to_string(d->reservoir.n ? 1 : 0) +
                       // whether the particles leave the list form among the candidates
-                      (lists_cap(d) ? "L" : "");
+                      (lists_cap(d) ? "L" : "") +
+                      // the forms' times depend on the particles each in its own way: 30 cubed voxels, K = 16,
+                      // with 250 particles lists 8.4 us per frame, stream 13.4; 80 cubed with 128,000 in place
+                      // 47, stream 100; the propensities' precision changes the cost of every reaction event
+                      "," + std::to_string(d->T.precision) + "," + std::to_string(64 - __builtin_clzll(d->p_max | 1ull));
     for (const RepDesc& r : d->h_reps) key += "|" + std::to_string(r.X) + "x" + std::to_string(r.Y) + "x" + std::to_string(r.Z);
     {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
         if (it != cache.end()) {
             if (d->cfg_index != it->second.first) {
-                settle(d);
-                CS_CUDA(cudaStreamSynchronize(d->stream));
                 d->seg_len = 0;
                 set_cfg(d, it->second.first);
             }
@@ -2371,8 +2375,6 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         }
     }
     if (frames == 0) frames = 1;
-    settle(d);
-    CS_CUDA(cudaStreamSynchronize(d->stream));
     const uint64_t p0 = d->p_max;  // frames of a trial may refresh it
     const size_t bytes = (size_t)d->total_voxels * d->K;
     struct Kept {
