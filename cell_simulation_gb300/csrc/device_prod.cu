@@ -547,6 +547,66 @@ static bool resident_fits(const DeviceProd* d);
 static bool inplace_fits(const DeviceProd* d);
 static bool fused_fits(const DeviceProd* d);
 
+// How the fused stream and the in-place form divide a handle's lattices: bitmap words, the stream's groups (a
+// warp each) and the blocks of the in-place form's X and Y launches.
+struct Shape {
+    uint64_t words = 0, groups = 0, xb = 0, yb = 0;
+};
+
+// log2 of the word columns of an X (a = 0) or Y unit: as many as the unit may list while its launch still has
+// several blocks for every SM (line_target words).
+static uint64_t line_target(const DeviceProd* d) {
+    return std::min<uint64_t>(INPLACE_LINE_WORDS, d->occ_words / ((uint64_t)d->num_sms * 3));
+}
+static uint32_t line_columns(const RepDesc& r, int a) { return a == 0 ? r.Y * r.Wz : r.Wz; }
+static uint32_t line_lw(const RepDesc& r, int a, uint64_t target) {
+    const uint32_t len = a == 0 ? r.X : r.Y;
+    uint32_t lw = 0;
+    while ((1u << lw) < line_columns(r, a) && ((uint64_t)len << (lw + 1)) <= target) lw++;
+    return lw;
+}
+
+static Shape shape_of(const DeviceProd* d) {
+    Shape s;
+    const uint64_t target = line_target(d);
+    for (const RepDesc& r : d->h_reps) {
+        s.words += (uint64_t)r.X * r.Y * r.Wz;
+        s.groups += r.Wz <= 32 ? (uint64_t)r.X * ((r.Y + 32u / r.Wz - 1u) / (32u / r.Wz)) : (uint64_t)r.X * r.Y * ((r.Wz + 31u) / 32u);
+        for (int a = 0; a < 2; a++) {
+            const uint32_t lw = line_lw(r, a, target);
+            (a == 0 ? s.xb : s.yb) += (a == 0 ? 1u : r.X) * (uint64_t)((line_columns(r, a) + (1u << lw) - 1u) >> lw);
+        }
+    }
+    return s;
+}
+
+// Whether the in-place form is the faster of the two where there are more than few or sparse particles (us per
+// frame, stream / in place).  It touches less, but a line's block waits for its fullest column, and the stream's
+// warps catch up once they fill the chip:
+//  - fewer than 8 voxels per word leave both mostly empty words, and in place has more of them to scan (200 x 200 x 1
+//    with 80,000 particles 35 / 44, 800 x 800 x 6 with 384,000 91 / 119; 300 x 300 x 9 with 405,000 95 / 86), fewer
+//    than 20 once the chip is full (800 x 800 x 16 with 1 M 145 / 172);
+//  - few blocks, each a chain of its own: fewer than 24 of 512 words or more (1000 x 16 x 16 with 64,000 47 / 80; 16 of 16
+//    words, 16 cubed with 16,000, 90 / 40), or fewer than one per SM with 14,000 particles each (30 x 700 x 30 with
+//    157,500 102 / 77, with 945,000 502 / 643 in the 12-species network);
+//  - warps that fill the chip: more than 2.2 M particles and particles times groups past 1.8e10 (150 cubed: 1.7 M 278 /
+//    190, 3.4 M 594 / 580, 6.8 M 972 / 1132; 200 cubed: 2 M 214 / 211, 8 M 648 / 807; 250 cubed: 1.6 M 215 / 160, 6.3 M
+//    607 / 656);
+//  - replicates past 3,000 groups: as a Y block is never more than a plane, it needs planes of 160 words, and at most 2 M
+//    particles (8 replicates of 60 .. 70 cubed with 100,000 each 195 / 101; 128 of 16 .. 32 cubed with 1,500 71 / 82, with
+//    20,000 489 / 620; 512 of 16 .. 32 with 1,500 116 / 193; 64 of 64 .. 96 with 1,500 118 / 98, 60 of 60 .. 70 with 100,000
+//    576 / 753).
+static bool inplace_pays(const DeviceProd* d) {
+    const Shape s = shape_of(d);
+    const uint64_t p = d->p_max * d->n_rep, blocks = std::min(s.xb, s.yb);
+    const bool full = s.groups > 30ull * (uint64_t)d->num_sms;  // the stream holds 24 warps per SM
+    if (d->total_voxels < (full ? 20 : 8) * s.words) return false;
+    if (blocks < 24u && s.words >= 512u * blocks) return false;
+    if (blocks < (uint64_t)d->num_sms && p > 14000u * blocks) return false;
+    if (d->n_rep > 1u) return s.groups <= 3000u || (s.words >= 160u * s.yb && p <= 2000000u);
+    return p <= 2200000u || (double)p * (double)s.groups <= 1.8e10;
+}
+
 // Default step before any autotuning (us per frame in runs of 200, and of a call of one frame):
 //  - few particles per replicate (fewer than four replicates: up to 512 at K = 8, 256 at K = 16, as its one block is
 //    then the longer chain; stream / lists, 57 x 47 x 3 with 400 particles 13.4 / 8.6, with 800 14.0 / 13.8
@@ -556,33 +616,43 @@ static bool fused_fits(const DeviceProd* d);
 //    hash but loads the lattice in each call (64 x 64 x 1, 400 particles: resident 5.4 / 14.3, lists 8.3 /
 //    14.1; 109 x 52 x 1, 200 particles: 4.2 / 16.7 against 5.9 / 12.7), up to 1,280 particles
 //    at K = 8, 640 at K = 16 (64 x 64 x 1, K = 16, 1,000 particles, call of two: 52, stream 43);
+//  - a reaction without reactants, or reservoirs: every voxel, or many, run the SSA in each frame, and the in-place form
+//    spreads them over all warps (stream / in place, reaction without reactants: 64 x 64 x 1 53 / 19, 32 cubed 1514 / 47, 150
+//    cubed 2947 / 1746, 256 cubed 8078 / 7950; 256 replicates of 16 .. 32 cubed 3026 / 2459, 128 of 48 .. 64 10817 / 12185;
+//    reservoirs in a fiftieth of the voxels: 32 cubed 87 / 18, 150 cubed 138 / 68, 200 cubed with 8 M particles 931 / 979;
+//    with 1 voxel per word 64 x 64 x 1 15 / 16, 200 x 200 x 1 30 / 34);
 //  - up to 2.5 M voxels in all: few or sparse particles the fused sweep stream, whose frame is two dependent
 //    launches against the in-place form's three (stream / in place: 64^3 with 5,000 particles 18.4 / 25.9,
 //    130^3 with 12,000 29.8 / 28.2 and 75 / 77 in a call of two frames, 170^3 with 3,000 30.1 / 24.0; two
 //    fifths of a particle per voxel at most: 20 x 17 x 24 with half of one 34.8 / 25.5).  With one region:
 //    up to 14,336 particles, or one in ten voxels (the 12-species network: 64^3 with 12,000 23.9 / 32.0, with
-//    28,000 38.7 / 35.2, 80^3 with 30,000 33.3 / 36.1, with 60,000 56.9 / 40.2).  Several regions gather
+//    28,000 38.7 / 35.2, 80^3 with 30,000 33.3 / 36.1, with 60,000 56.9 / 40.2), and up to 4.4 M voxels one in
+//    twelve (160^3 with 205,000 62 / 72, with 410,000 93 / 86; K = 8 with 330,000 70 / 74; 168^3 with 237,000 63 / 58).  Several regions gather
 //    particles in some, and the fullest group sets a pass's time: up to 6,144, or one in 24 voxels (100^3 with
 //    32,000 33.7 / 32.8, 61 x 97 x 45 with 16,000 46.6 / 34.2);
-//  - else the in-place sweep stream;
-//  - rows or edges too long for that: the fused sweep stream at three blocks per SM, or four-block sweep
+//  - else the in-place sweep stream where it pays (inplace_pays);
+//  - else, or with rows or edges too long for that, the fused sweep stream at three blocks per SM, or four-block sweep
 //    passes and a three-block pass 3.
 static constexpr uint64_t RESIDENT_DEFAULT_VOXELS = 4608;
-static constexpr uint64_t STREAM_DEFAULT_VOXELS = 2500000;
+static constexpr uint64_t STREAM_DEFAULT_VOXELS = 2500000, STREAM_DEFAULT_VOXELS_ONE = 4400000;
 static int pick_default_cfg(const DeviceProd* d, bool lists) {
     if (lists && lists_cap(d)) {
         const bool small = d->n_rep <= (uint32_t)d->num_sms && max_rep_voxels(d) <= RESIDENT_DEFAULT_VOXELS;
         if (small && d->p_max * d->K <= 10240u && resident_fits(d)) return find_cfg(d->K, KIND_RESIDENT, 0);
         if (d->n_rep >= 4u || d->p_max * d->K <= 4096u) return find_cfg(d->K, KIND_LISTS, 0);
     }
-    const int stream = find_cfg(d->K, KIND_STREAM, fused_fits(d) ? 4 : 2);
+    const int stream = find_cfg(d->K, KIND_STREAM, fused_fits(d) ? 4 : 2), inplace = find_cfg(d->K, KIND_INPLACE, 0);
     if (!inplace_fits(d)) return stream;
-    if (d->total_voxels <= STREAM_DEFAULT_VOXELS) {
-        const uint64_t V = d->total_voxels, p = d->p_max * d->n_rep;
-        const bool one = d->NC <= 2u;  // one region code beside the outside's
+    const uint64_t V = d->total_voxels, p = d->p_max * d->n_rep;
+    if (d->T.n_zero_order && (d->n_rep == 1u || V <= 8000000u)) return inplace;
+    if (d->reservoir.n && V >= 8u * d->occ_words && p <= 4000000u) return inplace;
+    const bool one = d->NC <= 2u;  // one region code beside the outside's
+    if (V <= STREAM_DEFAULT_VOXELS) {
         if ((p <= (one ? 14336u : 6144u) && 5 * p <= 2 * V) || (one ? 10 : 24) * p <= V) return stream;
+    } else if (d->n_rep == 1u && one && V <= STREAM_DEFAULT_VOXELS_ONE && p >= 20000u && 12 * p <= V) {
+        return stream;
     }
-    return find_cfg(d->K, KIND_INPLACE, 0);
+    return inplace_pays(d) ? inplace : stream;
 }
 
 // The region code shared by every lattice voxel of brick w's region window
@@ -761,15 +831,13 @@ static void build_units(DeviceProd* d) {
         d->unit_off[a].assign(d->n_rep + 1, 0);
         d->unit_words[a] = 1;
     }
-    const uint64_t line_target = std::min<uint64_t>(INPLACE_LINE_WORDS, d->occ_words / ((uint64_t)d->num_sms * 3));
+    const uint64_t target = line_target(d);
     const uint64_t row_target = std::min<uint64_t>(INPLACE_ROW_WORDS, d->occ_words / ((uint64_t)d->num_sms * 6) + 1);
     for (uint32_t ri = 0; ri < d->n_rep; ri++) {
         const RepDesc& r = d->h_reps[ri];
         for (int a = 0; a < 3; a++) d->unit_off[a][ri] = (uint32_t)u[a].size();
         for (int a = 0; a < 2; a++) {
-            const uint32_t len = a == 0 ? r.X : r.Y, cols = a == 0 ? r.Y * r.Wz : r.Wz;
-            uint32_t lw = 0;
-            while ((1u << lw) < cols && ((uint64_t)len << (lw + 1)) <= line_target) lw++;
+            const uint32_t len = a == 0 ? r.X : r.Y, cols = line_columns(r, a), lw = line_lw(r, a, target);
             d->unit_words[a] = std::max(d->unit_words[a], len << lw);
             for (uint32_t l = 0; l < (a == 0 ? 1u : r.X); l++)
                 for (uint32_t c = 0; c < cols; c += 1u << lw) {
