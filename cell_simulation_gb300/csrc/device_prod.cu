@@ -240,7 +240,12 @@ struct DeviceProd {
     uint32_t* h_flag = nullptr;
     bool ls_state = false;
     uint64_t p_max = 0;
-    cudaEvent_t piece_ev[2] = {};  // ends of the last two launches of a long call
+    // auto_form: the form is the default rule's choice (for p_pick particles), and follows the population
+    bool auto_form = false;
+    bool source = false;  // a reaction takes nothing away: the population may grow without bound
+    uint64_t p_pick = 0;
+    cudaEvent_t piece_ev[2] = {};  // ends of the last two pieces of a long call
+    unsigned long long* h_piece = nullptr;  // pinned: the counts at those
     DevBuf<uint32_t> ip_from;      // InplaceParams::from while replicates are brought to one frame, else empty
     DevBuf<uint32_t> exchange;  // workspace of lattice uploads and read-backs (see exchange_piece)
     uint32_t one_code = 0;  // the region code of every voxel of a single lattice when they share one, else 0
@@ -281,6 +286,7 @@ struct DeviceProd {
             if (g1) cudaGraphExecDestroy(g1);
         if (h_counts) cudaFreeHost(h_counts);
         if (h_flag) cudaFreeHost(h_flag);
+        if (h_piece) cudaFreeHost(h_piece);
         if (h_frames) cudaFreeHost(h_frames);
         for (cudaEvent_t e : frame_ev)
             if (e) cudaEventDestroy(e);
@@ -331,6 +337,7 @@ static void build_tables(DeviceProd* d, const Model& m) {
             cdl[8 * r + n] = (int8_t)v;
             n++;
         }
+        if (n > 0 && *std::min_element(&cdl[8 * r], &cdl[8 * r] + n) > 0) d->source = true;
     }
     if (d->R > 128) throw Error(CS_ERR_LIMIT, "at most 128 reactions on the production path");
     // candidate masks: bit r of rmask[s] when s is a reactant of reaction r
@@ -546,6 +553,7 @@ static uint64_t max_rep_voxels(const DeviceProd* d);
 static bool resident_fits(const DeviceProd* d);
 static bool inplace_fits(const DeviceProd* d);
 static bool fused_fits(const DeviceProd* d);
+static void set_cfg(DeviceProd* d, int idx);
 
 // How the fused stream and the in-place form divide a handle's lattices: bitmap words, the stream's groups (a
 // warp each) and the blocks of the in-place form's X and Y launches.
@@ -653,6 +661,17 @@ static int pick_default_cfg(const DeviceProd* d, bool lists) {
         return stream;
     }
     return inplace_pays(d) ? inplace : stream;
+}
+
+// Takes the form that the rule gives for the particles as they are, lists and the resident form among the
+// candidates unless `lists` is false.
+static void take_default(DeviceProd* d, bool lists) {
+    d->auto_form = true;
+    d->p_pick = d->p_max;
+    const int idx = pick_default_cfg(d, lists);
+    if (idx == d->cfg_index) return;
+    CS_CUDA(cudaStreamSynchronize(d->stream));
+    set_cfg(d, idx);
 }
 
 // The region code shared by every lattice voxel of brick w's region window
@@ -1467,7 +1486,7 @@ DeviceProd* prod_create(const Model& m, int device) {
         CS_CUDA(cudaMemcpy(d->resv_bits.p, rb.data(), rb.size() * 4, cudaMemcpyHostToDevice));
     }
     prod_set_lattice(d.get(), m, m.slots.data());
-    set_cfg(d.get(), pick_default_cfg(d.get(), true));
+    take_default(d.get(), true);
     return d.release();
 }
 
@@ -1863,43 +1882,88 @@ static bool run_lists(DeviceProd* d, uint32_t n, bool batched) {
     return true;
 }
 
-// n frames of the list form in launches of LIST_MAX_FRAMES; while one runs the host looks whether the launch
-// before has stopped, so that at most two launches are made in vain.  Returns the frames that were not
-// enqueued: the particles have outgrown the lists.
-static uint32_t run_list_pieces(DeviceProd* d, uint32_t n, bool batched) {
-    uint32_t pieces = 0;
-    while (n) {
-        const uint32_t m = std::min(n, LIST_MAX_FRAMES);
-        if (!run_lists(d, m, batched)) return n;
-        n -= m;
-        if (n == 0) break;
-        cudaEvent_t& ev = d->piece_ev[pieces & 1u];
-        if (!ev) CS_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        CS_CUDA(cudaEventRecord(ev, d->stream));
-        if (pieces) CS_CUDA(cudaEventSynchronize(d->piece_ev[(pieces & 1u) ^ 1u]));
-        pieces++;
-    }
-    return 0;
-}
-
 static bool lists_stopped(const DeviceProd* d) { return d->ls_state && *static_cast<volatile uint32_t*>(d->h_flag) != 0u; }
 
-// Enqueues n frames; the frame number must already be in stepbuf[cur] (and
-// its host copy in next_frame).  Where lists have stopped, the frames that they
-// lack come first; with hold they do not, nothing more is enqueued, and the
-// stream is idle: returns whether that is so.
-static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold) {
-    if (n == 0) return false;
-    while (all_cfgs()[d->cfg_index].kind == KIND_LISTS) {
-        n = run_list_pieces(d, n, batched);
-        if (n == 0) return false;
-        CS_CUDA(cudaStreamSynchronize(d->stream));
-        if (hold && lists_stopped(d)) return true;
-        if (!lists_settle(d)) set_cfg(d, pick_default_cfg(d, false));
+static uint64_t most_particles(const DeviceProd* d, const unsigned long long* counts) {
+    uint64_t most = 0;
+    for (size_t r = 0; r < d->n_rep; r++) {
+        uint64_t p = 0;
+        for (uint32_t s = 1; s < d->S1; s++) p += counts[r * d->S1 + s];
+        most = std::max(most, p);
     }
+    return most;
+}
+
+// The form follows the population where the rule chose it: the rule is asked again once the particles that the
+// host knows of have changed by half.
+static bool population_changed(const DeviceProd* d) {
+    return d->auto_form && (2u * d->p_max > 3u * d->p_pick || 3u * d->p_max < 2u * d->p_pick);
+}
+
+// After a piece of a long call: its counts start on their way, and those of the piece before are read, so that
+// the GPU always has a piece to run.
+static void watch_piece(DeviceProd* d, uint32_t piece) {
+    const size_t n = (size_t)d->n_rep * d->S1;
+    if (!d->h_piece) CS_CUDA(cudaMallocHost(&d->h_piece, 2 * n * 8));
+    cudaEvent_t& ev = d->piece_ev[piece & 1u];
+    if (!ev) CS_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    CS_CUDA(cudaMemcpyAsync(d->h_piece + (piece & 1u) * n, d->counts.p, n * 8, cudaMemcpyDeviceToHost, d->stream));
+    CS_CUDA(cudaEventRecord(ev, d->stream));
+    if (piece == 0) return;
+    CS_CUDA(cudaEventSynchronize(d->piece_ev[(piece & 1u) ^ 1u]));
+    d->p_max = most_particles(d, d->h_piece + ((piece & 1u) ^ 1u) * n);
+}
+
+static void run_piece(DeviceProd* d, uint32_t n, bool batched);
+
+// Enqueues n frames; the frame number must already be in stepbuf[cur] (and
+// its host copy in next_frame).  A long call in lists, or in a form of the
+// rule's choice, goes piece by piece: the host looks between the pieces whether
+// lists have stopped and what the particles have become.  Where lists have
+// stopped, the frames that they lack come first; with hold they do not, nothing
+// more is enqueued, and the stream is idle: returns whether that is so.
+static constexpr uint32_t RESIDENT_PIECE = 256, RESIDENT_PIECE_SOURCE = 128;  // a launch's start and end: 1% of 128 frames
+static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold) {
+    uint32_t watched = 0;  // pieces since the call began or lists stopped
+    while (n) {
+        if (population_changed(d) && d->ls_state) CS_CUDA(cudaStreamSynchronize(d->stream));
+        if (hold && lists_stopped(d)) {
+            CS_CUDA(cudaStreamSynchronize(d->stream));
+            return true;
+        }
+        if (population_changed(d)) {
+            settle(d);
+            try {
+                take_default(d, true);
+            } catch (const OutOfMemory&) {  // the form that it has goes on
+            }
+        }
+        const int kind = all_cfgs()[d->cfg_index].kind;
+        uint32_t m = n;
+        if (kind == KIND_LISTS) {
+            m = std::min(n, LIST_MAX_FRAMES);
+            if (!run_lists(d, m, batched)) {
+                CS_CUDA(cudaStreamSynchronize(d->stream));
+                if (hold && lists_stopped(d)) return true;
+                if (!lists_settle(d)) take_default(d, false);
+                watched = 0;
+                continue;
+            }
+        } else {
+            const uint32_t most = kind != KIND_RESIDENT ? LIST_MAX_FRAMES : d->source ? RESIDENT_PIECE_SOURCE : RESIDENT_PIECE;
+            if (d->auto_form && n >= 2u * most) m = most;
+            run_piece(d, m, batched);
+        }
+        n -= m;
+        if (n) watch_piece(d, watched++);
+    }
+    return false;
+}
+
+static void run_piece(DeviceProd* d, uint32_t n, bool batched) {
     if (all_cfgs()[d->cfg_index].kind == KIND_INPLACE) {
         run_inplace(d, n, batched);
-        return false;
+        return;
     }
     ensure_slots(d);
     d->ip_state = d->ip_valid = d->ls_state = false;
@@ -1909,7 +1973,7 @@ static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold
         d->next_frame += n;
         d->occ_valid = false;  // the resident form keeps no occupancy bitmaps and no x-decisions
         d->xdec_valid = false;
-        return false;
+        return;
     }
     // the brick pass and the sweep stream read and maintain the occupancy bitmaps
     const int kind = all_cfgs()[d->cfg_index].kind;
@@ -1989,7 +2053,6 @@ static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold
         d->xdec_frame = d->next_frame;
         d->xdec_epoch = d->seed_epoch;
     }
-    return false;
 }
 
 // The frame number of the next frame into stepbuf[cur] (the step's one
@@ -2017,12 +2080,7 @@ static void fetch_counts(DeviceProd* d) {
     if (!d->h_counts) CS_CUDA(cudaMallocHost(&d->h_counts, (n + 1) * 8));
     CS_CUDA(cudaMemcpyAsync(d->h_counts, d->counts.p, (n + 1) * 8, cudaMemcpyDeviceToHost, d->stream));
     CS_CUDA(cudaStreamSynchronize(d->stream));
-    d->p_max = 0;
-    for (size_t r = 0; r < d->n_rep; r++) {
-        uint64_t p = 0;
-        for (uint32_t s = 1; s < d->S1; s++) p += d->h_counts[r * d->S1 + s];
-        d->p_max = std::max(d->p_max, p);
-    }
+    d->p_max = most_particles(d, d->h_counts);
 }
 
 // After a stop, with the stream idle: the handle goes back to the earliest frame at which a replicate stands
@@ -2045,7 +2103,9 @@ static void lists_leave(DeviceProd* d) {
         const bool longer = lists_cap(d) > d->l_cap;
         ensure_slots(d);
         d->ls_state = false;
-        set_cfg(d, pick_default_cfg(d, longer));
+        set_cfg(d, pick_default_cfg(d, longer));  // longer lists are laid out anew, too
+        d->auto_form = true;
+        d->p_pick = d->p_max;
     } else {
         ensure_slots(d);
         d->ls_state = false;
@@ -2078,8 +2138,7 @@ static bool lists_settle(DeviceProd* d) {
                 continue;
             }
             fetch_counts(d);
-            const int idx = pick_default_cfg(d, true);
-            if (idx != d->cfg_index) set_cfg(d, idx);
+            take_default(d, true);
         }
         return true;
     }
@@ -2088,8 +2147,7 @@ static bool lists_settle(DeviceProd* d) {
     d->ip_from.reset();
     drop_graphs(d);
     fetch_counts(d);
-    const int idx = pick_default_cfg(d, lists_cap(d) > cap);
-    if (idx != d->cfg_index) set_cfg(d, idx);
+    take_default(d, lists_cap(d) > cap);
     return true;
 }
 
@@ -2292,7 +2350,7 @@ DeviceProd* prod_ensemble_create(const Model& m, uint32_t n, const uint32_t* res
     CS_CUDA(cudaMemcpy(d->counts.p, cnt.data(), cnt.size() * 8, cudaMemcpyHostToDevice));
     d->cur = 0;
     for (uint32_t s = 1; s < d->S1; s++) d->p_max += init_counts[s];
-    set_cfg(d.get(), pick_default_cfg(d.get(), true));
+    take_default(d.get(), true);
     return d.release();
 }
 
@@ -2337,6 +2395,7 @@ void prod_set_tiling(DeviceProd* d, int cfg_index, uint32_t seg_len) {
     d->seg_len = seg_len;
     try {
         set_cfg(d, cfg_index);
+        d->auto_form = false;
     } catch (...) {
         d->seg_len = keep;  // a refused variant leaves the handle as it was
         throw;
@@ -2434,6 +2493,7 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
         if (it != cache.end()) {
+            d->auto_form = false;
             if (d->cfg_index != it->second.first) {
                 d->seg_len = 0;
                 set_cfg(d, it->second.first);
@@ -2475,11 +2535,13 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
     };
     const int cfg0 = d->cfg_index;
     const uint32_t seg0 = d->seg_len;
+    const bool auto0 = d->auto_form;
     const auto& c = all_cfgs();
     int best = -1;
     float best_t = 0.0f;
     save(start);
     try {
+        d->auto_form = false;  // trials keep their variant
         size_t free_bytes = 0, all_bytes = 0;
         CS_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
         // room for the copy beside every variant's buffers (112 bytes per voxel of a bitmap word: the
@@ -2519,7 +2581,10 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
                 restore();
                 if (rep == 0 || r < t) t = r;
             }
-            if (d->cfg_index != i) continue;  // the particles outgrew the lists, and other forms were timed
+            if (d->cfg_index != i) {  // the particles outgrew the lists, and other forms were timed
+                d->auto_form = false;
+                continue;
+            }
             if (best < 0 || t < best_t) { best = i; best_t = t; }
         }
         if (best < 0) throw Error(CS_ERR_LIMIT, "no step variant can be set up for this lattice");
@@ -2533,6 +2598,7 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
             restore();
             d->seg_len = seg0;
             set_cfg(d, cfg0);
+            d->auto_form = auto0;
         } catch (...) {
         }
         throw;

@@ -1,13 +1,13 @@
 """The form that the default rule takes on both sides of the lines that decide between the fused sweep stream and
-the in-place form on crowded, thin, long and many lattices.  Every run is compared bit for bit with the column
-tiles (the general path) or the oracle."""
+the in-place form on crowded, thin, long and many lattices, and how a handle of the rule's choice follows its
+population.  Every run is compared bit for bit with the column tiles (the general path) or the oracle."""
 import numpy as np
 import pytest
 
 from cell_simulation_gb300 import Ensemble, RNG_PHILOX, configs, tiling_kinds, tiling_variants
 from cell_simulation_gb300.simulation import LatticeParams, Simulation
 from tests.helpers import LAM, multi_region_model
-from tests.test_new_forms_gpu import one_region
+from tests.test_new_forms_gpu import in_place, lists, one_region
 from tests.test_prod_gpu import oracle_prod
 
 pytestmark = pytest.mark.gpu
@@ -124,3 +124,49 @@ def test_replicates(n, edge, particles, want):
         ens.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("K", [8, 16])
+def test_form_follows_an_upload(K):
+    """A handle made with few particles takes the form of the lattice that is uploaded, and back; one whose variant
+    was chosen keeps it."""
+    few, many = mixed((16, 16, 16), K, 100), mixed((16, 16, 16), K, 16000)
+    outs = []
+    for tiling in (None, tiles(K), in_place(K)):
+        sim = few()
+        sim.prepare_for_gpu(RNG_PHILOX, 0)
+        if tiling is not None:
+            sim.set_tiling(tiling)
+        seen = [sim.get_tiling()]
+        got = []
+        for mk in (many, few, many):
+            sim.set_lattice(mk().get_lattice()[0])
+            sim.step_philox(7, 3)
+            seen.append(sim.get_tiling())
+            got += [sim.get_lattice()[0], sim.counts()]
+        outs.append(got)
+        if tiling is None:
+            assert [form(t) for t in seen] == [RESIDENT, IN_PLACE, RESIDENT, IN_PLACE]
+        else:
+            assert seen == [tiling] * 4
+    for a, b, c in zip(*outs):
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+
+
+def test_form_follows_a_population_that_grows(orc):
+    """Grown within one long call, and within calls whose counts are read."""
+    mk = lambda: one_region((64, 64, 1), 8, (20, 0, 0), (30.0, 10.0, 20.0))
+    want = oracle_prod(orc, mk(), 2048, seed=7)
+    assert want[1].sum() > 15000
+    for calls in ((2048,), (256,) * 8):
+        sim = mk()
+        sim.prepare_for_gpu(RNG_PHILOX, 0)
+        assert form(sim.get_tiling()) == RESIDENT
+        for n in calls:
+            sim.step_philox(n, 7)
+            if len(calls) > 1:
+                sim.counts()
+        assert np.array_equal(sim.get_lattice()[0].astype(np.uint8), want[0])
+        assert np.array_equal(sim.counts(), want[1])
+        assert np.array_equal(sim.diagnostics()[:4], want[2][:4])
+        assert form(sim.get_tiling()) == STREAM
