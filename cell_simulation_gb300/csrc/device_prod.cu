@@ -243,6 +243,7 @@ struct DeviceProd {
     // auto_form: the form is the default rule's choice (for p_pick particles), and follows the population
     bool auto_form = false;
     bool source = false;  // a reaction takes nothing away: the population may grow without bound
+    bool stream_beside = false;  // the fused stream's work lists were made after the last set_cfg (run_stream_call)
     uint64_t p_pick = 0;
     cudaEvent_t piece_ev[2] = {};  // ends of the last two pieces of a long call
     unsigned long long* h_piece = nullptr;  // pinned: the counts at those
@@ -623,7 +624,8 @@ static bool inplace_pays(const DeviceProd* d) {
 //    / 13.8 and 48 / 54): the list form; or, up to 4,608 voxels, the resident form, which needs no
 //    hash but loads the lattice in each call (64 x 64 x 1, 400 particles: resident 5.4 / 14.3, lists 8.3 /
 //    14.1; 109 x 52 x 1, 200 particles: 4.2 / 16.7 against 5.9 / 12.7), up to 1,280 particles
-//    at K = 8, 640 at K = 16 (64 x 64 x 1, K = 16, 1,000 particles, call of two: 52, stream 43);
+//    at K = 8, 640 at K = 16 (64 x 64 x 1, K = 16, 1,000 particles, call of two: 52, stream 43); its short calls
+//    are the stream's (resident_call);
 //  - a reaction without reactants, or reservoirs: every voxel, or many, run the SSA in each frame, and the in-place form
 //    spreads them over all warps (stream / in place, reaction without reactants: 64 x 64 x 1 53 / 19, 32 cubed 1514 / 47, 150
 //    cubed 2947 / 1746, 256 cubed 8078 / 7950; 256 replicates of 16 .. 32 cubed 3026 / 2459, 128 of 48 .. 64 10817 / 12185;
@@ -1091,6 +1093,7 @@ static void set_cfg(DeviceProd* d, int idx) {
         throw;
     }
     drop_graphs(d);
+    d->stream_beside = false;
 }
 
 // Occupancy bitmap of one replicate's slot buffer: one warp per (x, y) row,
@@ -1900,6 +1903,12 @@ static bool population_changed(const DeviceProd* d) {
     return d->auto_form && (2u * d->p_max > 3u * d->p_pick || 3u * d->p_max < 2u * d->p_pick);
 }
 
+// Whether a call of n frames of a handle in the resident form is that form's: it loads and stores the lattice in
+// each call, so that a short call of many particles is faster in the fused stream (us of a call of 1 / 2 / 5 frames on
+// 64 x 64 x 1, K = 8, stream and resident: 400 particles 25 / 38 / 76 and 25 / 37 / 50, 640 25 / 38 / 79 and 29 / 39 /
+// 66, 1,024 25 / 39 / 84 and 37 / 50 / 87; 16^3, K = 16, 640 38 / 51 / 113 and 37 / 50 / 99).
+static bool resident_call(const DeviceProd* d, uint32_t n) { return !d->auto_form || d->p_max <= 200ull * (n + 1ull); }
+
 // After a piece of a long call: its counts start on their way, and those of the piece before are read, so that
 // the GPU always has a piece to run.
 static void watch_piece(DeviceProd* d, uint32_t piece) {
@@ -1915,6 +1924,25 @@ static void watch_piece(DeviceProd* d, uint32_t piece) {
 }
 
 static void run_piece(DeviceProd* d, uint32_t n, bool batched);
+
+// A short call of a handle in the resident form (resident_call): the fused stream's work lists stand beside it, as the
+// resident form has none of its own.
+static void run_stream_call(DeviceProd* d, uint32_t n, bool batched) {
+    const int resident = d->cfg_index;
+    d->cfg_index = find_cfg(d->K, KIND_STREAM, fused_fits(d) ? 4 : 2);
+    try {
+        if (!d->stream_beside) {
+            set_attrs(d, all_cfgs()[d->cfg_index]);
+            build_groups(d);
+            d->stream_beside = true;
+        }
+        run_piece(d, n, batched);
+    } catch (...) {
+        d->cfg_index = resident;
+        throw;
+    }
+    d->cfg_index = resident;
+}
 
 // Enqueues n frames; the frame number must already be in stepbuf[cur] (and
 // its host copy in next_frame).  A long call in lists, or in a form of the
@@ -1968,6 +1996,10 @@ static void run_piece(DeviceProd* d, uint32_t n, bool batched) {
     ensure_slots(d);
     d->ip_state = d->ip_valid = d->ls_state = false;
     if (all_cfgs()[d->cfg_index].kind == KIND_RESIDENT) {
+        if (!resident_call(d, n)) {
+            run_stream_call(d, n, batched);
+            return;
+        }
         launch_resident(d, n, batched);
         d->cur ^= (int)(n & 1u);
         d->next_frame += n;

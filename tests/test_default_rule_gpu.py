@@ -1,6 +1,7 @@
 """The form that the default rule takes on both sides of the lines that decide between the fused sweep stream and
 the in-place form on crowded, thin, long and many lattices, and how a handle of the rule's choice follows its
-population.  Every run is compared bit for bit with the column tiles (the general path) or the oracle."""
+population and the length of its calls.  Every run is compared bit for bit with the column tiles (the general
+path) or the oracle."""
 import numpy as np
 import pytest
 
@@ -124,6 +125,12 @@ def test_replicates(n, edge, particles, want):
         ens.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("K,particles", [(8, 400), (8, 401), (8, 900), (16, 640)])
+def test_short_calls_of_a_resident_handle(K, particles):
+    """Calls of one frame up to twenty, in the stream or in the resident form, one after another."""
+    check(mixed((64, 64, 1), K, particles), K, RESIDENT, calls=(1, 1, 2, 5, 1, 20, 3, 1, 4, 2, 2))
 
 
 @pytest.mark.parametrize("K", [8, 16])
