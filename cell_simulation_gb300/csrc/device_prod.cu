@@ -2277,7 +2277,9 @@ void prod_render_view(DeviceProd* d, int32_t view, int32_t slice_axis, uint32_t 
         if (lists_settle(d)) prod_render_view(d, view, slice_axis, slice, out_host, out_device);
         return;
     }
-    ensure_slots(d);
+    // views 1 and 2 read no slots: to write them first made a region view of 256^3 voxels, K = 16, after in-place frames
+    // 141 us instead of 94
+    if (view == 0) ensure_slots(d);
     ViewParams v{};
     v.slots = d->slots[d->cur].p;
     v.K = d->K;
