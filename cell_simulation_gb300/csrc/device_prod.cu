@@ -243,6 +243,9 @@ struct DeviceProd {
     // auto_form: the form is the default rule's choice (for p_pick particles), and follows the population
     bool auto_form = false;
     bool source = false;  // a reaction takes nothing away: the population may grow without bound
+    // p_bound: what p_max can grow to.  No reaction raises the counts' sum with these weights (empty: none found)
+    std::vector<uint64_t> weights;
+    uint64_t p_bound = ~0ull;
     bool stream_beside = false;  // the fused stream's work lists were made after the last set_cfg (run_stream_call)
     uint64_t p_pick = 0;
     cudaEvent_t piece_ev[2] = {};  // ends of the last two pieces of a long call
@@ -305,6 +308,31 @@ static uint32_t threshold_of(double D, double tau, double lambda) {
     return t >= 4294967295.0 ? 0xFFFFFFFFu : (uint32_t)t;
 }
 
+// DeviceProd::weights from the change lists: one each, raised on what a reaction takes away while the reaction would
+// raise the sum; empty when that does not end.
+static std::vector<uint64_t> population_weights(uint32_t R, uint32_t S1, const std::vector<uint8_t>& sp,
+                                                const std::vector<int8_t>& change) {
+    std::vector<uint64_t> w(S1, 1);
+    for (bool again = true; again;) {
+        again = false;
+        for (uint32_t r = 0; r < R; r++) {
+            int64_t gain = 0, taken = 0;
+            for (uint32_t i = 8 * r; i < 8 * r + 8; i++) {
+                gain += (int64_t)w[sp[i]] * change[i];
+                taken -= std::min<int64_t>(change[i], 0);
+            }
+            if (gain <= 0) continue;
+            if (taken == 0) return {};
+            const int64_t more = (gain + taken - 1) / taken;
+            for (uint32_t i = 8 * r; i < 8 * r + 8; i++)
+                if (change[i] < 0) w[sp[i]] += (uint64_t)more;
+            if (*std::max_element(w.begin(), w.end()) > 64u) return {};
+            again = true;
+        }
+    }
+    return w;
+}
+
 // Builds the shared reaction/diffusion tables of the production path.
 static void build_tables(DeviceProd* d, const Model& m) {
     d->K = m.K;
@@ -340,6 +368,7 @@ static void build_tables(DeviceProd* d, const Model& m) {
         }
         if (n > 0 && *std::min_element(&cdl[8 * r], &cdl[8 * r] + n) > 0) d->source = true;
     }
+    d->weights = population_weights(d->R, d->S1, csp, cdl);
     if (d->R > 128) throw Error(CS_ERR_LIMIT, "at most 128 reactions on the production path");
     // candidate masks: bit r of rmask[s] when s is a reactant of reaction r
     std::vector<unsigned long long> rmask(2 * (size_t)d->S1, 0ull);
@@ -555,6 +584,23 @@ static bool resident_fits(const DeviceProd* d);
 static bool inplace_fits(const DeviceProd* d);
 static bool fused_fits(const DeviceProd* d);
 static void set_cfg(DeviceProd* d, int idx);
+
+// p_max and p_bound from the counts of n_rep replicates.
+static void set_population(DeviceProd* d, const unsigned long long* counts, size_t n_rep) {
+    uint64_t most = 0, bound = 0;
+    for (size_t r = 0; r < n_rep; r++) {
+        uint64_t p = 0, w = 0;
+        for (uint32_t s = 1; s < d->S1; s++) {
+            p += counts[r * d->S1 + s];
+            if (!d->weights.empty()) w += d->weights[s] * counts[r * d->S1 + s];
+        }
+        most = std::max(most, p);
+        bound = std::max(bound, w);
+    }
+    d->p_max = most;
+    // a reservoir's particle reacts without being used up
+    d->p_bound = d->weights.empty() || d->reservoir.n ? ~0ull : bound;
+}
 
 // How the fused stream and the in-place form divide a handle's lattices: bitmap words, the stream's groups (a
 // warp each) and the blocks of the in-place form's X and Y launches.
@@ -1614,8 +1660,7 @@ void prod_set_lattice(DeviceProd* d, const Model& m, const uint32_t* slots) {
     std::vector<unsigned long long> c(d->S1);
     CS_CUDA(cudaMemcpyAsync(c.data(), d->counts.p, c.size() * 8, cudaMemcpyDeviceToHost, d->stream));
     CS_CUDA(cudaStreamSynchronize(d->stream));
-    d->p_max = 0;
-    for (uint32_t s = 1; s < d->S1; s++) d->p_max += c[s];
+    set_population(d, c.data(), 1);
 }
 
 static void get_lattice_once(DeviceProd* d, const Model& m, uint32_t* slots, uint32_t* occ, int32_t* conc);
@@ -1887,16 +1932,6 @@ static bool run_lists(DeviceProd* d, uint32_t n, bool batched) {
 
 static bool lists_stopped(const DeviceProd* d) { return d->ls_state && *static_cast<volatile uint32_t*>(d->h_flag) != 0u; }
 
-static uint64_t most_particles(const DeviceProd* d, const unsigned long long* counts) {
-    uint64_t most = 0;
-    for (size_t r = 0; r < d->n_rep; r++) {
-        uint64_t p = 0;
-        for (uint32_t s = 1; s < d->S1; s++) p += counts[r * d->S1 + s];
-        most = std::max(most, p);
-    }
-    return most;
-}
-
 // The form follows the population where the rule chose it: the rule is asked again once the particles that the
 // host knows of have changed by half.
 static bool population_changed(const DeviceProd* d) {
@@ -1909,6 +1944,14 @@ static bool population_changed(const DeviceProd* d) {
 // 66, 1,024 25 / 39 / 84 and 37 / 50 / 87; 16^3, K = 16, 640 38 / 51 / 113 and 37 / 50 / 99).
 static bool resident_call(const DeviceProd* d, uint32_t n) { return !d->auto_form || d->p_max <= 200ull * (n + 1ull); }
 
+// Whether a long call goes piece by piece: the particles may grow until lists stop, or another form is the rule's
+// choice.  Other calls only enqueue, as the host would else wait for most of the call, and with it another handle's
+// calls (two handles of the 64 x 64 x 1 model stepped by one thread ran one after the other).
+static bool must_watch(const DeviceProd* d) {
+    if (d->auto_form && d->p_bound > d->p_pick + d->p_pick / 2u) return true;
+    return all_cfgs()[d->cfg_index].kind == KIND_LISTS && d->p_bound > d->l_cap / 2u;
+}
+
 // After a piece of a long call: its counts start on their way, and those of the piece before are read, so that
 // the GPU always has a piece to run.
 static void watch_piece(DeviceProd* d, uint32_t piece) {
@@ -1920,7 +1963,7 @@ static void watch_piece(DeviceProd* d, uint32_t piece) {
     CS_CUDA(cudaEventRecord(ev, d->stream));
     if (piece == 0) return;
     CS_CUDA(cudaEventSynchronize(d->piece_ev[(piece & 1u) ^ 1u]));
-    d->p_max = most_particles(d, d->h_piece + ((piece & 1u) ^ 1u) * n);
+    set_population(d, d->h_piece + ((piece & 1u) ^ 1u) * n, d->n_rep);
 }
 
 static void run_piece(DeviceProd* d, uint32_t n, bool batched);
@@ -1979,11 +2022,11 @@ static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold
             }
         } else {
             const uint32_t most = kind != KIND_RESIDENT ? LIST_MAX_FRAMES : d->source ? RESIDENT_PIECE_SOURCE : RESIDENT_PIECE;
-            if (d->auto_form && n >= 2u * most) m = most;
+            if (must_watch(d) && n >= 2u * most) m = most;
             run_piece(d, m, batched);
         }
         n -= m;
-        if (n) watch_piece(d, watched++);
+        if (n && must_watch(d)) watch_piece(d, watched++);
     }
     return false;
 }
@@ -2112,7 +2155,7 @@ static void fetch_counts(DeviceProd* d) {
     if (!d->h_counts) CS_CUDA(cudaMallocHost(&d->h_counts, (n + 1) * 8));
     CS_CUDA(cudaMemcpyAsync(d->h_counts, d->counts.p, (n + 1) * 8, cudaMemcpyDeviceToHost, d->stream));
     CS_CUDA(cudaStreamSynchronize(d->stream));
-    d->p_max = most_particles(d, d->h_counts);
+    set_population(d, d->h_counts, d->n_rep);
 }
 
 // After a stop, with the stream idle: the handle goes back to the earliest frame at which a replicate stands
@@ -2383,7 +2426,7 @@ DeviceProd* prod_ensemble_create(const Model& m, uint32_t n, const uint32_t* res
     d->occ_valid = false;
     CS_CUDA(cudaMemcpy(d->counts.p, cnt.data(), cnt.size() * 8, cudaMemcpyHostToDevice));
     d->cur = 0;
-    for (uint32_t s = 1; s < d->S1; s++) d->p_max += init_counts[s];
+    set_population(d.get(), cnt.data(), 1);  // the same in every replicate
     take_default(d.get(), true);
     return d.release();
 }
@@ -2537,7 +2580,7 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         }
     }
     if (frames == 0) frames = 1;
-    const uint64_t p0 = d->p_max;  // frames of a trial may refresh it
+    const uint64_t p0 = d->p_max, bound0 = d->p_bound;  // frames of a trial may refresh them
     const size_t bytes = (size_t)d->total_voxels * d->K;
     struct Kept {
         DevBuf<uint8_t> slots;
@@ -2566,6 +2609,7 @@ int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched,
         d->ip_state = d->ip_valid = d->ls_state = d->slots_stale = false;
         d->frame_known = false;
         d->p_max = p0;
+        d->p_bound = bound0;
     };
     const int cfg0 = d->cfg_index;
     const uint32_t seg0 = d->seg_len;
