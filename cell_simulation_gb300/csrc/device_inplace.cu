@@ -1087,10 +1087,10 @@ void region_windows(const uint8_t* rpad, const RepDesc& rd, uint8_t* wcode, uint
     CS_LAUNCH_CHECK();
 }
 
-void inplace_view(int K, const InplaceParams& P, const RepDesc& rd, float* out, cudaStream_t s) {
+void inplace_view(int K, const InplaceParams& P, const RepDesc& rd, uint32_t num_sms, float* out, cudaStream_t s) {
     const uint64_t words = (uint64_t)rd.X * rd.Y * rd.Wz;
     // words of a warp (at most 32, one per lane): few enough that small lattices still fill the chip
-    const uint64_t most = words / (152u * 32u) + 1u;
+    const uint64_t most = words / (num_sms * 32u) + 1u;
     const uint32_t per = most < 32u ? (uint32_t)most : 32u;
     const uint64_t blocks = (words + 8u * per - 1u) / (8u * per);
     const unsigned grid = (unsigned)(blocks < 4096u ? blocks : 4096u);

@@ -641,16 +641,16 @@ static Shape shape_of(const DeviceProd* d) {
 //  - fewer than 8 voxels per word leave both mostly empty words, and in place has more of them to scan (200 x 200 x 1
 //    with 80,000 particles 35 / 44, 800 x 800 x 6 with 384,000 91 / 119; 300 x 300 x 9 with 405,000 95 / 86), fewer
 //    than 20 once the chip is full (800 x 800 x 16 with 1 M 145 / 172);
-//  - few blocks, each a chain of its own: fewer than 24 of 512 words or more (1000 x 16 x 16 with 64,000 47 / 80; 16 of 16
-//    words, 16 cubed with 16,000, 90 / 40), or fewer than one per SM with 14,000 particles each (30 x 700 x 30 with
-//    157,500 102 / 77, with 945,000 502 / 643 in the 12-species network);
+//  - few blocks, each a chain of its own: fewer than 24 of 512 words or more (1000 x 16 x 16 with 64,000 47 / 80; 16
+//    of 16 words, 16 cubed with 16,000, 90 / 40), or fewer than one per SM with 14,000 particles each (30 x 700 x 30
+//    with 157,500 102 / 77, with 945,000 502 / 643 in the 12-species network);
 //  - warps that fill the chip: more than 2.2 M particles and particles times groups past 1.8e10 (150 cubed: 1.7 M 278 /
 //    190, 3.4 M 594 / 580, 6.8 M 972 / 1132; 200 cubed: 2 M 214 / 211, 8 M 648 / 807; 250 cubed: 1.6 M 215 / 160, 6.3 M
 //    607 / 656);
-//  - replicates past 3,000 groups: as a Y block is never more than a plane, it needs planes of 160 words, and at most 2 M
-//    particles (8 replicates of 60 .. 70 cubed with 100,000 each 195 / 101; 128 of 16 .. 32 cubed with 1,500 71 / 82, with
-//    20,000 489 / 620; 512 of 16 .. 32 with 1,500 116 / 193; 64 of 64 .. 96 with 1,500 118 / 98, 60 of 60 .. 70 with 100,000
-//    576 / 753).
+//  - replicates past 3,000 groups: as a Y block is never more than a plane, it needs planes of 160 words, and at most
+//    2 M particles (8 replicates of 60 .. 70 cubed with 100,000 each 195 / 101; 128 of 16 .. 32 cubed with 1,500 71 /
+//    82, with 20,000 489 / 620; 512 of 16 .. 32 with 1,500 116 / 193; 64 of 64 .. 96 with 1,500 118 / 98, 60 of 60 ..
+//    70 with 100,000 576 / 753).
 static bool inplace_pays(const DeviceProd* d) {
     const Shape s = shape_of(d);
     const uint64_t p = d->p_max * d->n_rep, blocks = std::min(s.xb, s.yb);
@@ -672,20 +672,20 @@ static bool inplace_pays(const DeviceProd* d) {
 //    14.1; 109 x 52 x 1, 200 particles: 4.2 / 16.7 against 5.9 / 12.7), up to 1,280 particles
 //    at K = 8, 640 at K = 16 (64 x 64 x 1, K = 16, 1,000 particles, call of two: 52, stream 43); its short calls
 //    are the stream's (resident_call);
-//  - a reaction without reactants, or reservoirs: every voxel, or many, run the SSA in each frame, and the in-place form
-//    spreads them over all warps (stream / in place, reaction without reactants: 64 x 64 x 1 53 / 19, 32 cubed 1514 / 47, 150
-//    cubed 2947 / 1746, 256 cubed 8078 / 7950; 256 replicates of 16 .. 32 cubed 3026 / 2459, 128 of 48 .. 64 10817 / 12185;
-//    reservoirs in a fiftieth of the voxels: 32 cubed 87 / 18, 150 cubed 138 / 68, 200 cubed with 8 M particles 931 / 979;
-//    with 1 voxel per word 64 x 64 x 1 15 / 16, 200 x 200 x 1 30 / 34);
-//  - up to 2.5 M voxels in all: few or sparse particles the fused sweep stream, whose frame is two dependent
-//    launches against the in-place form's three (stream / in place: 64^3 with 5,000 particles 18.4 / 25.9,
-//    130^3 with 12,000 29.8 / 28.2 and 75 / 77 in a call of two frames, 170^3 with 3,000 30.1 / 24.0; two
-//    fifths of a particle per voxel at most: 20 x 17 x 24 with half of one 34.8 / 25.5).  With one region:
-//    up to 14,336 particles, or one in ten voxels (the 12-species network: 64^3 with 12,000 23.9 / 32.0, with
-//    28,000 38.7 / 35.2, 80^3 with 30,000 33.3 / 36.1, with 60,000 56.9 / 40.2), and up to 4.4 M voxels one in
-//    twelve (160^3 with 205,000 62 / 72, with 410,000 93 / 86; K = 8 with 330,000 70 / 74; 168^3 with 237,000 63 / 58).  Several regions gather
-//    particles in some, and the fullest group sets a pass's time: up to 6,144, or one in 24 voxels (100^3 with
-//    32,000 33.7 / 32.8, 61 x 97 x 45 with 16,000 46.6 / 34.2);
+//  - a reaction without reactants, or reservoirs: every voxel, or many, run the SSA in each frame, and the in-place
+//    form spreads them over all warps (stream / in place, reaction without reactants: 64 x 64 x 1 53 / 19, 32 cubed
+//    1514 / 47, 150 cubed 2947 / 1746, 256 cubed 8078 / 7950; 256 replicates of 16 .. 32 cubed 3026 / 2459, 128 of 48
+//    .. 64 10817 / 12185; reservoirs in a fiftieth of the voxels: 32 cubed 87 / 18, 150 cubed 138 / 68, 200 cubed
+//    with 8 M particles 931 / 979; with 1 voxel per word 64 x 64 x 1 15 / 16, 200 x 200 x 1 30 / 34);
+//  - up to 2.5 M voxels in all: few or sparse particles the fused sweep stream, whose frame is two dependent launches
+//    against the in-place form's three (stream / in place: 64^3 with 5,000 particles 18.4 / 25.9, 130^3 with 12,000
+//    29.8 / 28.2 and 75 / 77 in a call of two frames, 170^3 with 3,000 30.1 / 24.0; two fifths of a particle per
+//    voxel at most: 20 x 17 x 24 with half of one 34.8 / 25.5).  With one region: up to 14,336 particles, or one in
+//    ten voxels (the 12-species network: 64^3 with 12,000 23.9 / 32.0, with 28,000 38.7 / 35.2, 80^3 with 30,000 33.3
+//    / 36.1, with 60,000 56.9 / 40.2), and up to 4.4 M voxels one in twelve (160^3 with 205,000 62 / 72, with 410,000
+//    93 / 86; K = 8 with 330,000 70 / 74; 168^3 with 237,000 63 / 58).  Several regions gather particles in some, and
+//    the fullest group sets a pass's time: up to 6,144, or one in 24 voxels (100^3 with 32,000 33.7 / 32.8, 61 x 97 x
+//    45 with 16,000 46.6 / 34.2);
 //  - else the in-place sweep stream where it pays (inplace_pays);
 //  - else, or with rows or edges too long for that, the fused sweep stream at three blocks per SM, or four-block sweep
 //    passes and a three-block pass 3.
@@ -1546,16 +1546,15 @@ void prod_destroy(DeviceProd* d) {
     delete d;
 }
 
-// Uploads a reference-layout lattice (u32 slots) for replicate 0, compacting
-// each voxel's slots, and resets the species counts to slots + reservoirs.
 // Bit 7 of every non-zero byte.
 __device__ __forceinline__ uint64_t nonzero_bytes(uint64_t x) {
     return (((x & 0x7F7F7F7F7F7F7F7Full) + 0x7F7F7F7F7F7F7F7Full) | x) & 0x8080808080808080ull;
 }
 
 // The caller's 32-bit slots of n voxels from v0 on into the device's bytes, particles first,
-// and their number by species (the callers have checked that they are species of the model).  One thread per voxel; bound by the host's copies on either side: 71,040 voxels
-// of K = 8 with 120,000 particles took 785 us here on the host (and 650 us the other way) for copies of 20 us.
+// and their number by species (the callers have checked that they are species of the model).  One thread per voxel;
+// bound by the host's copies on either side: 71,040 voxels of K = 8 with 120,000 particles took 785 us here on the
+// host (and 650 us the other way) for copies of 20 us.
 template <int K>
 __global__ void __launch_bounds__(256) import_slots_kernel(const uint4* in, uint64_t v0, uint32_t n, uint8_t* slots,
                                                            const uint8_t* reservoir,
@@ -1631,6 +1630,8 @@ static unsigned exchange_grid(const DeviceProd* d, uint64_t n) {
     return (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)d->num_sms * 16);
 }
 
+// Uploads a reference-layout lattice (u32 slots) for replicate 0, compacting
+// each voxel's slots, and resets the species counts to slots + reservoirs.
 void prod_set_lattice(DeviceProd* d, const Model& m, const uint32_t* slots) {
     DeviceGuard g(d->device);
     const uint64_t V = m.V, piece = exchange_piece(V, m.K);
@@ -1911,7 +1912,9 @@ static bool run_lists(DeviceProd* d, uint32_t n, bool batched) {
     P.n_frames = n;
     // more threads where SMs have at most one block anyway: fewer rounds of a sweep's entries and more warps
     // for the SSAs, against dearer barriers (us per frame with 512 / 768 threads, 96 replicates of the 12-species
-    // network on 12 .. 24 cubed voxels: 300 particles 11.5 / 11.9, 450 15.7 / 14.0, 600 20.0 / 19.1, 780 25.1 / 22.9)
+    // network on 12 .. 24 cubed voxels: 300 particles 11.5 / 11.9, 450 15.7 / 14.0, 600 20.0 / 19.1, 780 25.1 / 22.9).
+    // 256 where they hold the particles at once (256 / 512 threads, the same replicates: 100 particles 8.2 / 8.3, 128
+    // 9.1 / 9.0, 160 10.9 / 9.3; one lattice of 40 cubed voxels, K = 8: 100 6.5 / 6.6, 128 7.0 / 6.8, 160 8.7 / 7.2)
     const int threads = d->n_rep > (uint32_t)d->num_sms || d->p_max <= 128 ? 256 : d->p_max <= 350 ? 512 : 768;
     if (batched) {
         lists_launch((int)d->K, threads, P, d->n_rep, d->stream);
@@ -2314,14 +2317,14 @@ void prod_render_view(DeviceProd* d, int32_t view, int32_t slice_axis, uint32_t 
     if (view == 0 && slice == 0u && d->slots_stale) {
         // the form's own layout is read: far fewer bytes than writing the slots first
         if (d->ls_state) lists_view((int)d->K, lists_params(d), r, out_dev, d->stream);
-        else inplace_view((int)d->K, inplace_params(d), r, out_dev, d->stream);
+        else inplace_view((int)d->K, inplace_params(d), r, (uint32_t)d->num_sms, out_dev, d->stream);
         if (!out_device) CS_CUDA(cudaMemcpyAsync(out_host, out_dev, V * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
         CS_CUDA(cudaStreamSynchronize(d->stream));
         if (lists_settle(d)) prod_render_view(d, view, slice_axis, slice, out_host, out_device);
         return;
     }
-    // views 1 and 2 read no slots: to write them first made a region view of 256^3 voxels, K = 16, after in-place frames
-    // 141 us instead of 94
+    // views 1 and 2 read no slots: to write them first made a region view of 256^3 voxels, K = 16, after in-place
+    // frames 141 us instead of 94
     if (view == 0) ensure_slots(d);
     ViewParams v{};
     v.slots = d->slots[d->cur].p;

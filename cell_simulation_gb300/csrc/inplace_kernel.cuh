@@ -39,9 +39,12 @@
 // from the snapshots and stores it.  No other block touches those voxels or
 // their words.
 //
-// Invariants between launches: an empty voxel's slots are zero; mv of an axis
-// is zero except between the pass that decides and the sweep that uses it (the
-// sweep clears the words it has used); occ, mul, mv and react have no bits
+// Invariants between launches: a voxel's slots are valid only where mul is set
+// (a lone particle is its byte in spec, an empty voxel its clear bit in occ, and
+// what the slots of either hold is left over), so whoever wants slots has them
+// written first (inplace_unpack) or reads occ, mul and spec; mv of an axis is zero except
+// between the pass that decides and the sweep that uses it (the sweep clears the
+// words it has used); occ, mul, mv and react have no bits
 // outside the lattice.  The lattice may be up to 1024 voxels long along each
 // axis.
 //
@@ -125,6 +128,6 @@ void inplace_pack(int K, const InplaceParams& P, cudaStream_t s);
 void inplace_unpack(int K, const InplaceParams& P, cudaStream_t s);
 
 // View 0 (the majority species / 255) of a replicate without writing its slots.
-void inplace_view(int K, const InplaceParams& P, const RepDesc& rd, float* out, cudaStream_t s);
+void inplace_view(int K, const InplaceParams& P, const RepDesc& rd, uint32_t num_sms, float* out, cudaStream_t s);
 
 }  // namespace cellsim
