@@ -188,6 +188,7 @@ struct DeviceProd {
     unsigned long long h_zmask[2] = {0ull, 0ull};
     DevBuf<unsigned long long> counts;
     DevBuf<uint32_t> diag, counters, stepbuf;
+    bool ctr_batched = true;  // whether the last frame that used the work counters was batched (run_piece)
     DevBuf<WorkItem> items;      // batched order
     DevBuf<WorkItem> items_rep;  // grouped per replicate (plain launches)
     std::vector<uint32_t> rep_item_off;
@@ -2064,6 +2065,10 @@ static void run_piece(DeviceProd* d, uint32_t n, bool batched) {
     if (!brick) d->occ_valid = false;  // the tile pipeline does not keep the bitmaps
     if (kind == KIND_STREAM && !d->groups_sorted) sort_groups(d);
     d->xdec_valid = false;
+    // batched frames and frames of one replicate have counters of their own, and a frame clears those of the next
+    // parity: after an odd number of frames of the other sort they are not clear, and a frame would find no work left
+    if (d->ctr_batched != batched) CS_CUDA(cudaMemsetAsync(d->counters.p, 0, d->counters.bytes(), d->stream));
+    d->ctr_batched = batched;
     if (kind == KIND_STREAM && !xdec_ok) launch_stream_pass0(d);
     uint32_t k = 0;
     // the multi-frame form for calls of two or more frames; a single frame gains nothing from it
