@@ -241,6 +241,7 @@ struct DeviceProd {
     uint32_t* h_flag = nullptr;
     bool ls_state = false;
     uint64_t p_max = 0;
+    bool p_known = false;  // no frame has run since p_max was taken
     // auto_form: the form is the default rule's choice (for p_pick particles), and follows the population
     bool auto_form = false;
     bool source = false;  // a reaction takes nothing away: the population may grow without bound
@@ -599,6 +600,7 @@ static void set_population(DeviceProd* d, const unsigned long long* counts, size
         bound = std::max(bound, w);
     }
     d->p_max = most;
+    d->p_known = true;
     // a reservoir's particle reacts without being used up
     d->p_bound = d->weights.empty() || d->reservoir.n ? ~0ull : bound;
 }
@@ -1968,6 +1970,7 @@ static void watch_piece(DeviceProd* d, uint32_t piece) {
     if (piece == 0) return;
     CS_CUDA(cudaEventSynchronize(d->piece_ev[(piece & 1u) ^ 1u]));
     set_population(d, d->h_piece + ((piece & 1u) ^ 1u) * n, d->n_rep);
+    d->p_known = false;
 }
 
 static void run_piece(DeviceProd* d, uint32_t n, bool batched);
@@ -2000,6 +2003,7 @@ static void run_stream_call(DeviceProd* d, uint32_t n, bool batched) {
 static constexpr uint32_t RESIDENT_PIECE = 256, RESIDENT_PIECE_SOURCE = 128;  // a launch's start and end: 1% of 128 frames
 static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold) {
     uint32_t watched = 0;  // pieces since the call began or lists stopped
+    if (n) d->p_known = false;
     while (n) {
         if (population_changed(d) && d->ls_state) CS_CUDA(cudaStreamSynchronize(d->stream));
         if (hold && lists_stopped(d)) {
@@ -2558,7 +2562,7 @@ static constexpr uint32_t kSettleFrames = 64;
 int prod_autotune(DeviceProd* d, uint32_t frames, uint64_t frame0, bool batched, float* best_ms) {
     DeviceGuard g(d->device);
     settle(d);
-    fetch_counts(d);
+    if (!d->p_known) fetch_counts(d);
     static std::mutex mu;
     static std::map<std::string, std::pair<int, float>> cache;
     cudaDeviceProp prop{};
