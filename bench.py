@@ -285,6 +285,8 @@ def launches_per_frame(i):
 def launches_in_call(i, frames):
     """Kernel launches of one step call of `frames` frames with variant i (none for pass 0, which
     runs only when the x-decisions are stale)."""
+    if describe_variant(i).get("lists"):
+        return -(-frames // 1024)  # the list form's longest launch
     if describe_variant(i).get("multi_frame"):
         return 1
     return frames * launches_per_frame(i)
@@ -498,7 +500,7 @@ def main():
     achieved = alg_bytes / frame_s / 1e9
     desc = describe_variant(variant)
     kernels = frame_kernels(desc)
-    longest = "sweep_pass_kernel<5>" if "sweep_pass_kernel<5>" in kernels else (
+    longest = kernels[-1] if desc.get("in_place") else "sweep_pass_kernel<5>" if "sweep_pass_kernel<5>" in kernels else (
         "sweep_pass_kernel<3>" if "sweep_pass_kernel<3>" in kernels else kernels[0])
     traffic = profiled_traffic(longest, w.name)
     per_kernel = {k: profiled_traffic(k, w.name) for k in kernels}
@@ -533,6 +535,9 @@ def main():
                      "traffic": traffic, "peak_kind": peak_kind,
                      "algorithmic_bytes_per_launch": alg_bytes, "kernel": longest,
                      "achieved_over": "frame time (every launch of the frame)",
+                     "frac_of": "dense-equivalent bytes (2K + 1 per voxel and frame, what a step over the whole "
+                                "lattice moves); the in-place, list and resident forms do not read the whole "
+                                "lattice, so for them it is no roofline: dram_frac is the bandwidth they use",
                      # the persistent kernel runs every frame of a call in one launch: its bytes are
                      # per frame of that launch
                      "traffic_per": "frame" if desc.get("multi_frame") else "launch",

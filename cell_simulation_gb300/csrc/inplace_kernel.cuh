@@ -52,14 +52,17 @@
 // voxel (X 53k, Y 30k, Z+D about 35k cycles per block of the 256 cubed cell: X has
 // strided words); below about 100 cubed, the latency of three dependent launches,
 // 25 us per frame whatever the content, where the fused stream's two win.  Blocks:
-// 256 threads and up to 1024 words for X and Y (128 / 512 measured 89 us per frame
-// against 82 on the 256 cubed cell), 128 / 512 for Z+D, whose decision pass wants
-// its registers (7 blocks per SM).  One 16-byte content load per voxel of the
-// decision pass made that frame 136 us: hence the species bytes.  us per frame,
-// fused sweep stream / this form: 256 cubed multi-region cell, 1 M particles 140 /
-// 82; 192 cubed stiff network, 1 M particles 151 / 121; 57 x 43 x 39 with two particles per voxel
-// 119 / 68; one persistent launch with grid barriers between the sweeps was slower
-// throughout (140, 325 us on the first two), as a barrier costs 2.7k - 4.7k cycles.
+// 256 threads and up to 1024 words for X and Y (128 / 512 measured 106 us per frame
+// against 98 on the 256 cubed cell, 128 against 121 on the 192 cubed one), 128 / 512
+// for Z+D, whose decision pass wants its registers (7 blocks per SM).  One 16-byte
+// content load per voxel of the decision pass made the 256 cubed frame 1.6 times as
+// long: hence the species bytes.  us per frame in one call from frame 80 on (three
+// processes within 1), fused sweep stream / this form: 256 cubed multi-region cell,
+// 1 M particles 146 / 98; 192 cubed stiff network, 1 M particles 152 / 121 (194 / 137
+// in its first 18 frames, while the placed particles spread); three species, K = 8, 57
+// x 43 x 39 with two particles per voxel 199 / 96.  One persistent launch with grid
+// barriers between the sweeps was slower throughout (1.7 and 2.7 times on the first
+// two), as a barrier costs 2.7k - 4.7k cycles.
 #pragma once
 #include <cuda_runtime.h>
 

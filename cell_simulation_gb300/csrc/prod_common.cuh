@@ -514,9 +514,7 @@ __device__ __forceinline__ void vox_remove(Vox<K>& c, uint32_t s, uint32_t n) {
 // binary64) exactly as react_voxel_inline forms them.  The selected candidate
 // is the first whose running sum exceeds the target (a ballot).  An event's
 // change list is applied to the content, its species deltas added to s_delta
-// (shared) or, when that is null, to the global counts row g_counts.  The SSA of
-// one voxel with one event (GB300, the stiff 12-species network): 12.0k cycles
-// with the histogram and sums in shared memory.
+// (shared) or, when that is null, to the global counts row g_counts.
 template <int K>
 __device__ __forceinline__ bool react_voxel_warp(Vox<K>& c, uint32_t resv, uint32_t v, uint32_t frame, uint32_t k0,
                                                  uint32_t k1, float mult, const ProdTables& T, int32_t* s_delta,

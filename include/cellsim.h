@@ -298,8 +298,7 @@ cs_status cs_step_philox_timed(cs_sim* sim, uint32_t n_steps, uint64_t seed, flo
  * persistent form that runs every frame of a step call in one launch, TY = 0
  * the per-pass launches), or with TY = 2 its in-place form, which makes every
  * decision of a frame in one pass and sweeps only the voxels that change
- * (edges of at most 1024 voxels; the default for lattices the list form does
- * not take); kind 3 = resident form: one block of `threads`
+ * (edges of at most 1024 voxels); kind 3 = resident form: one block of `threads`
  * per replicate holds its lattice in shared memory for every frame of a step
  * call (TY = TZ = 0; about 5,300 voxels per replicate at K = 16 and 9,000 at
  * K = 8 at most: cs_set_tiling refuses larger lattices); kind 4 = list form:
@@ -309,14 +308,19 @@ cs_status cs_step_philox_timed(cs_sim* sim, uint32_t n_steps, uint64_t seed, flo
  * reactions without reactants: cs_set_tiling refuses others; a replicate whose
  * particles outgrow its list stops before the frame that might not fit, and the
  * library runs the frames it lacks in other forms when it next looks: during a
- * call of more than 1,024 frames, at the next call, or when the state is read).  A new handle takes the resident
- * form (small lattices), the list form or the in-place form.  Every variant
- * computes the same lattice.  cs_tiling_launches: kernel launches per frame
+ * call of more than 1,024 frames, at the next call, or when the state is read).
+ * A new handle takes the resident form (small lattices) or the list form where
+ * its particles are few, else the fused sweep stream (small, sparse, thin or
+ * very full lattices, many replicates) or the in-place form, and asks again once
+ * the particles have changed by half (after an upload, a read of the counts, or
+ * within a long call); a variant set by cs_set_tiling or cs_autotune stays.
+ * Every variant computes the same lattice.  cs_tiling_launches: kernel launches per frame
  * once a run is under way (the sweep stream: 3, or 2 where the Y and Z sweeps
  * are one launch, or 1 per step call in the persistent form; the last two need
  * Z <= 1024 and cs_set_tiling refuses them otherwise; the in-place form: 3;
- * the resident and list forms: 1 per step call).  No reference counterpart (the reference has one
- * fixed dispatch shape per shader). */
+ * the resident form: 1 per step call; the list form: 1 per 1,024 frames of a
+ * step call).  No reference counterpart (the reference has one fixed dispatch
+ * shape per shader). */
 cs_status cs_tiling_count(int32_t* n);
 cs_status cs_tiling_describe(int32_t index, int32_t* K, int32_t* TY, int32_t* TZ, int32_t* threads);
 cs_status cs_tiling_kind(int32_t index, int32_t* kind, int32_t* brick_planes);
@@ -326,8 +330,10 @@ cs_status cs_get_tiling(const cs_sim* sim, int32_t* index);
 /* Autotuner: times every compiled variant for this K on the handle's own
  * lattice (frames_per_trial frames each, from a device copy of the current
  * state, which is restored afterwards, so the simulation does not advance),
- * selects the fastest and caches the choice per model shape and device for
- * the life of the process.  chosen_index / ms_per_frame may be NULL. */
+ * selects the fastest and caches the choice per model shape, precision, binary
+ * order of the particles and device for the life of the process.  A variant
+ * that does not fit is no candidate; on an error state and variant are the
+ * caller's.  chosen_index / ms_per_frame may be NULL. */
 cs_status cs_autotune(cs_sim* sim, uint32_t frames_per_trial, int32_t* chosen_index, float* ms_per_frame);
 
 /* ---------------- checkpoint / resume ---------------- */
