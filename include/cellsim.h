@@ -197,7 +197,9 @@ cs_status cs_prepare_for_gpu(cs_sim* sim, int32_t rng_mode, int32_t device);
  * (start_error_buffer_readbacks, src/simulation.rs:391-418); write_freq 0
  * disables sampling.  Returns after the work is enqueued. */
 cs_status cs_step(cs_sim* sim, uint32_t n_steps, const uint32_t* itimes, uint32_t write_freq);
-/* Production path (CS_RNG_PHILOX): n_steps frames keyed by `seed`. */
+/* Production path (CS_RNG_PHILOX): n_steps frames keyed by `seed`.  Returns
+ * after the work is enqueued; a call of 256 frames or more whose particles can
+ * outgrow the handle's step form waits for all but its last frames. */
 cs_status cs_step_philox(cs_sim* sim, uint32_t n_steps, uint64_t seed, uint32_t write_freq);
 /* Precision form of the production path (cs_precision). */
 cs_status cs_set_precision(cs_sim* sim, int32_t precision);
