@@ -49,8 +49,8 @@
 // scattered accesses per listed voxel (100 cubed with 40,000 24.2, before
 // 51.9; 160 cubed with 200,000 47.1, before 84.6).  Calls of 20 frames and a
 // view of 128 cubed with 22,000 particles: 989 -> 424 us; of 10 frames and a
-// view of 256 cubed with 1 M: 2,856 -> 1,657 us (1,780 on another box, where the
-// first pass over a new upload takes 2,410).
+// view of 256 cubed with 1 M: 2,856 -> 1,657 us (1,780 and 2,030 with
+// the reaction networks of two other seeds).
 //
 // A voxel in neither act nor touch holds no particle and no species count, its slots
 // are compacted and its conc[v][0] is already 1, so the reaction pass leaves
