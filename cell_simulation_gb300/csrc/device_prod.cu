@@ -714,6 +714,20 @@ static int pick_default_cfg(const DeviceProd* d, bool lists) {
     return inplace_pays(d) ? inplace : stream;
 }
 
+// Takes form idx.  Where the device has no room for its buffers, the form that the handle has goes on, or, in place of
+// lists, which may not hold the particles any more, the tile pipeline, which works in the two slot buffers.
+static void set_form(DeviceProd* d, int idx) {
+    try {
+        set_cfg(d, idx);
+    } catch (const OutOfMemory&) {
+        if (d->cfg_index < 0) throw;
+        if (all_cfgs()[d->cfg_index].kind != KIND_LISTS) return;
+        int tiles = 0;
+        while (all_cfgs()[tiles].kind != KIND_TILE || all_cfgs()[tiles].K != (int)d->K) tiles++;
+        set_cfg(d, tiles);
+    }
+}
+
 // Takes the form that the rule gives for the particles as they are, lists and the resident form among the
 // candidates unless `lists` is false.
 static void take_default(DeviceProd* d, bool lists) {
@@ -722,7 +736,7 @@ static void take_default(DeviceProd* d, bool lists) {
     const int idx = pick_default_cfg(d, lists);
     if (idx == d->cfg_index) return;
     CS_CUDA(cudaStreamSynchronize(d->stream));
-    set_cfg(d, idx);
+    set_form(d, idx);
 }
 
 // The region code shared by every lattice voxel of brick w's region window
@@ -892,6 +906,17 @@ static bool inplace_fits(const DeviceProd* d) {
     return true;
 }
 
+// The in-place form's buffers that grow with the lattice.
+static void reserve_inplace(DeviceProd* d) {
+    for (int a = 0; a < 3; a++) {
+        if (d->mv[a].n < d->occ_words) d->mv[a].alloc(d->occ_words);
+        if (d->dec[a].n < d->total_voxels) d->dec[a].alloc(d->total_voxels);
+    }
+    if (d->mul.n < d->occ_words) d->mul.alloc(d->occ_words);
+    if (d->spec.n < 32 * d->occ_words) d->spec.alloc(32 * d->occ_words);
+    if (d->react.n < d->occ_words) d->react.alloc(d->occ_words);
+}
+
 // Units of the in-place form's launches.  An X or Y unit takes whole lines of 2^lw word columns, a Z
 // unit whole rows; each is as large as its block can list (INPLACE_LINE_WORDS, INPLACE_ROW_WORDS)
 // while the launch still has several blocks for every SM.
@@ -935,12 +960,8 @@ static void build_units(DeviceProd* d) {
         d->unit_off[a][d->n_rep] = (uint32_t)u[a].size();
         d->units[a].alloc(u[a].size());
         CS_CUDA(cudaMemcpy(d->units[a].p, u[a].data(), u[a].size() * sizeof(LineUnit), cudaMemcpyHostToDevice));
-        if (d->mv[a].n < d->occ_words) d->mv[a].alloc(d->occ_words);
-        if (d->dec[a].n < d->total_voxels) d->dec[a].alloc(d->total_voxels);
     }
-    if (d->mul.n < d->occ_words) d->mul.alloc(d->occ_words);
-    if (d->spec.n < 32 * d->occ_words) d->spec.alloc(32 * d->occ_words);
-    if (d->react.n < d->occ_words) d->react.alloc(d->occ_words);
+    reserve_inplace(d);
     d->n_items = (uint32_t)u[2].size();
     d->ip_valid = false;
     ensure_wcode(d);
@@ -1135,10 +1156,16 @@ static void set_cfg(DeviceProd* d, int idx) {
     d->cfg_index = idx;
     try {
         build_items(d);
-        if (idx == d->refuse_cfg) throw Error(d->refuse_status, "variant refused by cs_debug_refuse_tiling");
+        if (idx == d->refuse_cfg) {
+            if (d->refuse_status == CS_ERR_CAPACITY) throw OutOfMemory(CS_ERR_CUDA, "no room, says cs_debug_refuse_tiling");
+            throw Error(d->refuse_status, "variant refused by cs_debug_refuse_tiling");
+        }
     } catch (...) {
         d->cfg_index = prev;
-        if (prev >= 0) build_items(d);
+        try {
+            if (prev >= 0) build_items(d);
+        } catch (const Error&) {  // lists that the particles have outgrown: run_lists takes another form
+        }
         throw;
     }
     drop_graphs(d);
@@ -2012,10 +2039,7 @@ static bool run_frames_nosync(DeviceProd* d, uint32_t n, bool batched, bool hold
         }
         if (population_changed(d)) {
             settle(d);
-            try {
-                take_default(d, true);
-            } catch (const OutOfMemory&) {  // the form that it has goes on
-            }
+            take_default(d, true);
         }
         const int kind = all_cfgs()[d->cfg_index].kind;
         uint32_t m = n;
@@ -2190,10 +2214,11 @@ static void lists_leave(DeviceProd* d) {
         const bool longer = lists_cap(d) > d->l_cap;
         ensure_slots(d);
         d->ls_state = false;
-        set_cfg(d, pick_default_cfg(d, longer));  // longer lists are laid out anew, too
+        set_form(d, pick_default_cfg(d, longer));  // longer lists are laid out anew, too
         d->auto_form = true;
         d->p_pick = d->p_max;
     } else {
+        reserve_inplace(d);  // while nothing has changed: a caller who makes room can go on
         ensure_slots(d);
         d->ls_state = false;
         set_cfg(d, find_cfg(d->K, KIND_INPLACE, 0));

@@ -230,7 +230,8 @@ cs_status cs_synchronize(cs_sim* sim);
 cs_status cs_debug_stall_group(cs_sim* sim, uint32_t group);
 /* Test hook of what happens when a step variant cannot be set up: cs_set_tiling
  * and the autotuner's trials of variant `index` fail with `status` from now on,
- * after its work lists have been made (index -1: none fails).  No reference
+ * after its work lists have been made (index -1: none fails; CS_ERR_CAPACITY: as
+ * when the device has no room for the variant's buffers, CS_ERR_CUDA).  No reference
  * counterpart. */
 cs_status cs_debug_refuse_tiling(cs_sim* sim, int32_t index, cs_status status);
 
